@@ -221,9 +221,9 @@ template <int L> struct StagedTw {
   }
 };
 
-// Fill a staged table from the flat one (flat[m] = e^{-2 pi i m/L}); all
-// threads of the CTA, published by the caller's next barrier.
-template <int L>
+// Fill a staged table from the flat one (flat[m STRIDE] = e^{-2 pi i m/L});
+// all threads of the CTA, published by the caller's next barrier.
+template <int L, int STRIDE = 1>
 __device__ __forceinline__ void staged_tw_build(double2 *dst, const double2 *__restrict__ flat) {
   using ST = StagedTw<L>;
   using RX = Radices<L>;
@@ -241,7 +241,7 @@ __device__ __forceinline__ void staged_tw_build(double2 *dst, const double2 *__r
       }
       off += 3 * ns;
     }
-    dst[i] = found ? flat[k * (1 << e) * (L / (ns * 8))] : make_double2(1.0, 0.0);
+    dst[i] = found ? flat[k * (1 << e) * (L / (ns * 8)) * STRIDE] : make_double2(1.0, 0.0);
   }
 }
 

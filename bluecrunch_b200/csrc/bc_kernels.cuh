@@ -23,7 +23,8 @@
 //                 8 consecutive coefficients -> (H, C), value H + C*2^{8b}
 //   k_carry       decoupled-lookback scan of run carries -> output words
 //
-// k_small does all of it in one CTA for M <= 4096.
+// k_small does all of it in one CTA for M <= 5120, k_cluster (bc_cluster.cuh)
+// in one cluster of CTAs.
 //
 // Reference correspondence: the whole pipeline computes what _fft_mul
 // computes (bigfloat/mul.c:108-174): the exact C = A*B mod 2^{32 CL}.
@@ -128,6 +129,11 @@ __device__ __forceinline__ double2 outer_tw(const Tw2 &T, int s, int k) {
   return tw2_get(T, (uint64_t)s * (uint64_t)(4 * k - 1));
 }
 
+// Nearest integer of |z| < 2^51 (ties to even, as rint): added to 1.5 2^52 the
+// fraction is rounded off.  Above that the result stays near z, so the check
+// below still sees a value too large.
+__device__ __forceinline__ double round_near(double z) { return (z + 6755399441055744.0) - 6755399441055744.0; }
+
 // Rounding check of one point: max |x - round(x)| of its two coefficients,
 // or 1.0 when a coefficient reaches 2^50 — beyond that the distance to the
 // nearest integer stops measuring the error (doubles near 2^53 hold no
@@ -149,46 +155,72 @@ __device__ __forceinline__ void atomic_max_err(unsigned long long *p, double e) 
 }
 
 // ------------------------------------------------------------------ runs
-// 8 consecutive rounded coefficients c_u (exact integers held in doubles) ->
-// H = sum (bits of the running carry) and C = final signed carry.
-// h |= bits << off for off < 192 (selects instead of a runtime word index,
-// so h stays in registers).
-__host__ __device__ __forceinline__ void u192_or_bits(U192 &h, unsigned long long bits, int off) {
-  const int wi = off >> 6, bi = off & 63;
-  const unsigned long long lo = bits << bi, hi = bi ? bits >> (64 - bi) : 0ull;
-  h.w[0] |= wi == 0 ? lo : 0ull;
-  h.w[1] |= wi == 1 ? lo : (wi == 0 ? hi : 0ull);
-  h.w[2] |= wi == 2 ? lo : (wi == 1 ? hi : 0ull);
+// Low 32 bits of (hi:lo) >> s and high 32 bits of (hi:lo) << s, 0 <= s < 32.
+__host__ __device__ __forceinline__ uint32_t shf_r(uint32_t lo, uint32_t hi, int s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_r(lo, hi, s);
+#else
+  return (uint32_t)((((unsigned long long)hi << 32) | lo) >> s);
+#endif
+}
+__host__ __device__ __forceinline__ uint32_t shf_l(uint32_t lo, uint32_t hi, int s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, s);
+#else
+  return (uint32_t)(((((unsigned long long)hi << 32) | lo) << s) >> 32);
+#endif
 }
 
+// An integer held in a double, |c| < 2^51, as 64 bits: added to 1.5 2^52 it
+// sits in the low bits of the sum (one add and one subtraction instead of
+// the conversion instruction, whose rate is a quarter of theirs).
+__host__ __device__ __forceinline__ long long int_of(double c) {
+#ifdef __CUDA_ARCH__
+  return __double_as_longlong(c + 6755399441055744.0) - 0x4338000000000000ll;
+#else
+  return (long long)c;
+#endif
+}
+
+// 8 consecutive rounded coefficients c_u (exact integers held in doubles) ->
+// H = sum (bits of the running carry) and C = final signed carry.  The digits
+// cut from the running carry (b <= 24 bits each) are packed from the top down,
+// H = H 2^b + digit, on 32-bit words: only the words that can be nonzero after
+// so many digits are shifted.
 __host__ __device__ __forceinline__ RunRec make_run(const double *c, int b) {
-  if (b == 16) {
-    // 8 x 16 bits fill two words exactly: constant shifts, no selects
-    unsigned long long h0 = 0, h1 = 0;
-    long long acc = 0;
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      acc += (long long)c[u];
-      const unsigned long long bits = (unsigned long long)acc & 0xffffull;
-      if (u < 4) h0 |= bits << (16 * u);
-      else h1 |= bits << (16 * (u - 4));
-      acc >>= 16;
-    }
-    RunRec r;
-    r.h0 = h0; r.h1 = h1; r.h2 = 0; r.c = acc;
-    return r;
-  }
-  U192 h = {{0, 0, 0}};
-  long long acc = 0;
-  const unsigned long long mask = (1ull << b) - 1;
+  uint32_t d[8];
+  uint32_t lo = 0, hi = 0;  // the running carry, signed 64 bits
+  const uint32_t mask = (1u << b) - 1;
 #pragma unroll
   for (int u = 0; u < 8; u++) {
-    acc += (long long)c[u];
-    u192_or_bits(h, (unsigned long long)acc & mask, b * u);
-    acc >>= b;  // arithmetic: floor division
+    const unsigned long long acc =
+        (((unsigned long long)hi << 32) | lo) + (unsigned long long)int_of(c[u]);
+    lo = (uint32_t)acc;
+    hi = (uint32_t)(acc >> 32);
+    d[u] = lo & mask;
+    lo = shf_r(lo, hi, b);
+    hi = (uint32_t)((int32_t)hi >> b);  // arithmetic: floor division
   }
   RunRec r;
-  r.h0 = h.w[0]; r.h1 = h.w[1]; r.h2 = h.w[2]; r.c = acc;
+  r.c = (long long)(((unsigned long long)hi << 32) | lo);
+  if (b == 16) {  // constant places
+    r.h0 = (unsigned long long)(d[0] | d[1] << 16) | (unsigned long long)(d[2] | d[3] << 16) << 32;
+    r.h1 = (unsigned long long)(d[4] | d[5] << 16) | (unsigned long long)(d[6] | d[7] << 16) << 32;
+    r.h2 = 0;
+    return r;
+  }
+  uint32_t w[6] = {d[7], 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int u = 6; u >= 0; u--) {
+    const int top = (24 * (8 - u) - 1) / 32;  // highest word after this digit
+#pragma unroll
+    for (int k = 5; k > 0; k--)
+      if (k <= top) w[k] = shf_l(w[k - 1], w[k], b);
+    w[0] = w[0] << b | d[u];
+  }
+  r.h0 = (unsigned long long)w[1] << 32 | w[0];
+  r.h1 = (unsigned long long)w[3] << 32 | w[2];
+  r.h2 = (unsigned long long)w[5] << 32 | w[4];
   return r;
 }
 
@@ -256,17 +288,22 @@ constexpr int LOOKBACK_SPINS = 1 << 22;
 __device__ __forceinline__ U192 rec_h(const RunRec &r) { U192 h = {{r.h0, r.h1, r.h2}}; return h; }
 
 // Words of run r (bits [r nbits, (r+1) nbits)) below nwords; a word that
-// straddles into run r+1 takes its high bits from hn.
+// straddles into run r+1 takes its high bits from hn.  nbits >= 64, so a run
+// starts 2 to 6 words.
 __device__ __forceinline__ void write_run_words(uint32_t *C, unsigned long long nwords, unsigned long long r,
                                                 int nbits, const U192 &h, const U192 &hn) {
   const unsigned long long bit0 = r * (unsigned long long)nbits;
-  unsigned long long w = (bit0 + 31) >> 5;
-  const unsigned long long wend = (bit0 + nbits + 31) >> 5;
-  for (; w < wend && w < nwords; w++) {
-    const int off = (int)((w << 5) - bit0);
-    uint32_t x = u192_bits32(h, off);
-    if (off + 32 > nbits) x |= u192_bits32(hn, 0) << (nbits - off);
-    C[w] = x;
+  const unsigned long long w0 = (bit0 + 31) >> 5;
+  const int o = (int)((w0 << 5) - bit0);  // bit of the run where word w0 starts, below 32
+  const uint32_t W[7] = {(uint32_t)h.w[0], (uint32_t)(h.w[0] >> 32), (uint32_t)h.w[1], (uint32_t)(h.w[1] >> 32),
+                         (uint32_t)h.w[2], (uint32_t)(h.w[2] >> 32), 0u};
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const int off = o + 32 * k;
+    if (off >= nbits || w0 + k >= nwords) break;
+    uint32_t x = shf_r(W[k], W[k + 1], o);
+    if (off + 32 > nbits) x |= (uint32_t)hn.w[0] << (nbits - off);
+    C[w0 + k] = x;
   }
 }
 
