@@ -137,10 +137,13 @@ constexpr int PTS = 8;
 // Montgomery, "Division by invariant integers using multiplication",
 // PLDI 1994, fig. 4.1): for 1 <= d < 2^32, l = ceil(log2 d),
 // m = floor(2^32 (2^l - d) / d) + 1, q = (t + ((n - t) >> min(l,1))) >> max(l-1,0)
-// with t = mulhi(m, n).  Built once per CTA; exact for every n < 2^32.
+// with t = mulhi(m, n); exact for every n < 2^32.  Built on the host and
+// passed with the kernel's parameters: its 64-bit division takes a thread 330
+// cycles, at the start of every CTA.
 struct FastDiv {
   uint32_t d, m;
   int s1, s2;
+  FastDiv() = default;
   __host__ __device__ explicit FastDiv(uint32_t div) : d(div) {
     int l = 0;
     while (l < 32 && (1ull << l) < (unsigned long long)div) l++;

@@ -747,7 +747,7 @@ KInfo get_fused(int L2, bool sq) {
 // items' A and B buffers are the contiguous slabs slabA / slabB (item i at
 // i*M).  Scratch (records, lookback status, counter) must be set up and the
 // counter and status words zeroed by the caller.
-int launch_class(const Shape &s, bool sq, const ClassParams &p, long long n, unsigned long long carry_tiles,
+int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n, unsigned long long carry_tiles,
                  double2 *slabA, double2 *slabB, cudaStream_t stream, bool timed, size_t *nl,
                  cudaEvent_t b_ready = nullptr, bool w16 = false, bool pdl_ok = false) {
   int r;
@@ -761,11 +761,19 @@ int launch_class(const Shape &s, bool sq, const ClassParams &p, long long n, uns
     // 2,750 limbs (8 CTAs each) 47 against 58 us, 64 of them 70 against 57;
     // 32 of 230 limbs 13 against 16 us, 64 of them 19 against 16.
     const KInfo kc = get_cluster(s.M, sq);
-    return launch(n * kc.cluster <= 2 * g.sm_count ? kc : get_small(s.M, sq), n, p, nl, stream, timed);
+    return launch(n * kc.cluster <= 2 * g.sm_count ? kc : get_small(s.M, sq), n, params, nl, stream, timed);
   }
-  const cuuint64_t M16 = (cuuint64_t)s.M * 16, S1 = (cuuint64_t)p.S1, Lr = (cuuint64_t)p.Lr;
+  const cuuint64_t M16 = (cuuint64_t)s.M * 16, S1 = (cuuint64_t)params.S1, Lr = (cuuint64_t)params.Lr;
   KInfo ko = get_outer(s.L1, false), ki = get_outer(s.L1, true);
   const int W1 = ko.threads / (s.L1 / ko.pts);
+  ClassParams p = params;
+  p.fd_outer = FastDiv((uint32_t)(S1 / W1));
+  p.fd_rows = FastDiv((uint32_t)(s.M / Lr));
+  if (s.levels == 3) {
+    const KInfo km = get_mid(s.L2, false);
+    p.fd_mid = FastDiv((uint32_t)(Lr / (km.threads / (s.L2 / km.pts))));
+    p.fd_op = FastDiv((uint32_t)s.L1 * p.fd_mid.d);
+  }
   // forward operands: every item's A, then the B slab's slots (items sharing
   // a B share a slot)
   const long long nb = sq ? 0 : (long long)p.nb;

@@ -54,17 +54,22 @@ __device__ __forceinline__ void dft_small16(double2 (&x)[R]) {
   else dft16<INV>(x);
 }
 
-// Shared-memory twiddles of block16: tw[t*16 + k2] = e^{-2 pi i t k2 / L},
-// t < L/16, k2 < 16, from the flat table flat[m] = e^{-2 pi i m/L}
-// (m < 3L/4; above that e^{-2 pi i m/L} = -e^{-2 pi i (m - L/2)/L}).  All
-// threads; the caller's next barrier publishes the table.
-template <int L>
+// Shared-memory twiddles of block16: tw[k2*R + t] = e^{-2 pi i t k2 / L},
+// t < R = L/16, k2 < 16, from the flat table flat[m] = e^{-2 pi i m/L}
+// (m < 3L/4; above that e^{-2 pi i m/L} = -e^{-2 pi i (m - L/2)/L}).  The
+// threads of a warp hold four or more neighbouring t of one k2: consecutive
+// entries, one pass over the banks (k2 fastest put them 256 bytes apart, four
+// passes).  All NT threads; the caller's next barrier publishes the table.
+template <int L, int NT>
 __device__ __forceinline__ void tw16_build(double2 *dst, const double2 *__restrict__ flat) {
-  for (int i = threadIdx.x; i < L; i += blockDim.x) {
-    const int m = (i >> 4) * (i & 15);
+  constexpr int R = L / P16;
+#pragma unroll
+  for (int q = 0; q < L / NT; q++) {
+    const int i = threadIdx.x + q * NT, m = (i % R) * (i / R);
     const double2 w = __ldg(&flat[m < 3 * L / 4 ? m : m - L / 2]);
     dst[i] = m < 3 * L / 4 ? w : make_double2(-w.x, -w.y);
   }
+  static_assert(L % NT == 0, "whole rounds");
 }
 
 // L-point transforms of W columns by R = L/16 threads per column.  On entry
@@ -76,7 +81,7 @@ __device__ __forceinline__ void block16(double2 (&v)[P16], int t, int s, double2
   constexpr int R = L / P16, J = P16 / R;
   dft16<INV>(v);  // v[k2] = Y[t][k2]
 #pragma unroll
-  for (int k2 = 1; k2 < P16; k2++) v[k2] = ctw<INV>(v[k2], tw[t * P16 + k2]);
+  for (int k2 = 1; k2 < P16; k2++) v[k2] = ctw<INV>(v[k2], tw[k2 * R + t]);
 #pragma unroll
   for (int k2 = 0; k2 < P16; k2++) sm[sidx<L, W>(k2 * R + t, s)] = v[k2];
   __syncthreads();
@@ -104,9 +109,9 @@ template <int L> struct Pass16 {
   static constexpr int MINB = 384 / NT;
   // dynamic shared memory
   static constexpr size_t TWB = (size_t)L * 16;  // block16 twiddles
-  static constexpr size_t SMEM_INV = 2 * (size_t)L * W * 16 + TWB + (size_t)L * 16 + 2 * 18 * 16 + 1024;
+  static constexpr size_t SMEM_INV = 2 * (size_t)L * W * 16 + TWB + (size_t)L * 16 + 2 * 36 * 16 + 1024;
   static constexpr size_t SMEM_FWD = (size_t)L * W * 16 + (size_t)PackTile<L>::STAGE_WORDS * 4 + TWB +
-                                     (size_t)L * 16 + 18 * 16 + 1024;
+                                     (size_t)L * 16 + 2 * 36 * 16 + 1024;
 };
 
 // Outer-pass twiddles e^{-2 pi i col (4 k1 - 1)/(4M)} of one thread, for
@@ -116,36 +121,42 @@ template <int L> struct Pass16 {
 //   base of the first run   T(col (4t - 1))     = F_t       * T(s (4t - 1))
 //   step                    T(col 4R)           = G         * T(s 4R)
 //   base of the second run  T(col (4t + 32R - 1)) = base1 * H * T(s 32R)
-// The tile factors F_t (t < 16), G = T(tile W 4R), H = T(tile W 32R) are
-// computed once per unit by 18 threads (sincospi) into shared memory; the
-// column factors depend only on the thread (s, t fixed by tid) and stay in
-// registers.  No global twiddle loads remain on the unit's path.
-constexpr int TILE_TW = 18;  // tile factors per unit
+// The tile factors F_t (t < 16), G = T(tile W 4R), H = T(tile W 32R) come
+// from the two-level table, T(m) = lo * hi: 18 threads copy both entries of
+// theirs to shared memory one unit ahead (cp.async), each thread multiplies
+// the three it needs.  The column factors depend only on the thread (s, t
+// fixed by tid) and stay in registers.  Computing the tile factors by
+// sincospi took 130 instructions in every warp of every unit, a tenth of the
+// pass's issue slots, and at the start of a CTA 2 us.
+constexpr int TILE_TW = 18;            // tile factors per unit
+constexpr int TILE_TW_N = 2 * TILE_TW;  // their table entries (lo, hi)
 
-// T(m) = e^{-2 pi i m/(4M)}: t4m(m, 2M) (bc_pipe.cuh).
+// Index of T(m) = e^{-2 pi i m/(4M)} in the two-level table, |m| < 4M.
+__device__ __forceinline__ unsigned long long t4m_index(long long m, int M) {
+  return (unsigned long long)(m < 0 ? m + 4ll * M : m);
+}
 
 struct ColTw16 {
   double2 c0, cst, cb1;
 };
 template <int R>
-__device__ __forceinline__ ColTw16 col_tw16(int s, int t, double twoM) {
+__device__ __forceinline__ ColTw16 col_tw16(int s, int t, const Tw2 &T, int M) {
   ColTw16 c;
-  c.c0 = t4m((long long)s * (4 * t - 1), twoM);
-  c.cst = t4m((long long)s * 4 * R, twoM);
-  c.cb1 = t4m((long long)s * 32 * R, twoM);
+  c.c0 = tw2_get(T, t4m_index((long long)s * (4 * t - 1), M));
+  c.cst = tw2_get(T, (unsigned long long)s * 4 * R);
+  c.cb1 = tw2_get(T, (unsigned long long)s * 32 * R);
   return c;
 }
 
-// The tile factors of `tile` into fac[0..17], spread over the CTA's warps
-// (a few lanes of each).  The caller's next barrier publishes them.
-template <int R, int W, int NT>
-__device__ __forceinline__ void tile_tw16(double2 *fac, int tile, double twoM) {
-  constexpr int NW = NT / 32, PER = (TILE_TW + NW - 1) / NW;
-  const int lane = threadIdx.x & 31, j = (threadIdx.x >> 5) * PER + lane;
-  if (lane < PER && j < TILE_TW) {
-    const long long tw = (long long)tile * W;
+// Copies the table entries of tile's factors to fac[0..35] (lo and hi of
+// factor j at 2j and 2j + 1); the caller commits, waits and synchronises.
+template <int R, int W>
+__device__ __forceinline__ void tile_tw16(double2 *fac, int tile, const Tw2 &T, int M) {
+  const int j = threadIdx.x >> 1;
+  if (j < TILE_TW) {
     const long long x = j < 16 ? 4 * j - 1 : (j == 16 ? 4 * R : 32 * R);
-    fac[j] = t4m(tw * x, twoM);
+    const unsigned long long m = t4m_index((long long)tile * W * x, M);
+    cp_async16(fac + threadIdx.x, (threadIdx.x & 1) ? &T.hi[m >> T.h] : &T.lo[m & T.mask], 16);
   }
 }
 
@@ -154,9 +165,9 @@ struct OuterRun16 {
 };
 __device__ __forceinline__ OuterRun16 outer_run16(const double2 *fac, const ColTw16 &c, int t) {
   OuterRun16 o;
-  o.b0 = cmul(fac[t], c.c0);
-  o.st = cmul(fac[16], c.cst);
-  o.b1 = cmul(o.b0, cmul(fac[17], c.cb1));
+  o.b0 = cmul(cmul(fac[2 * t], fac[2 * t + 1]), c.c0);
+  o.st = cmul(cmul(fac[32], fac[33]), c.cst);
+  o.b1 = cmul(o.b0, cmul(cmul(fac[34], fac[35]), c.cb1));
   return o;
 }
 
@@ -176,24 +187,22 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(C
   uint32_t *stg = reinterpret_cast<uint32_t *>(tile + L * W);  // one stage of STAGE_WORDS
   double2 *twS = reinterpret_cast<double2 *>(stg + K::STAGE_WORDS);
   double2 *pwS = twS + L;
-  double2 *fac = pwS + L;  // tile factors of the current unit
-  tw16_build<L>(twS, p.twL1);
-  table_to_smem(pwS, p.pw_fwd, L);
+  double2 *fac = pwS + L;  // tile factors of a unit, of the units in turn at fac + par * TILE_TW_N
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
-  const double twoM = 2.0 * (double)p.M;
-  const ColTw16 ct = col_tw16<R>(s, t, twoM);
-  const int tiles = p.S1 / W;
+  const int tiles = (int)p.fd_outer.d;
   const unsigned nA = fwd_units_a(p, (unsigned)tiles);
   const unsigned total = nA + fwd_units_b(p, (unsigned)tiles);  // far below 2^32
-  const FastDiv fd_tile((unsigned)tiles);
   // limb staging: as k2_outer_fwd (every row segment of a tile shares one
   // alignment below a 16-byte boundary)
   auto seg_shift = [&](int tl, int b, bool al16) -> int {
     return al16 ? (int)((((long long)tl * W * b >> 5) - 1) & 3) : 0;
   };
-  auto stage_copy = [&](unsigned u) {
-    const FwdUnit f = fwd_unit(p, u, nA, fd_tile, (unsigned)tiles);
+  // the unit's limb words and, to the set `par`, its tile factors (the threads
+  // still at the unit before read the other set)
+  auto stage_copy = [&](unsigned u, int par) {
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
     const int tl = (int)f.rest, op = f.op;
+    tile_tw16<R, W>(fac + par * TILE_TW_N, tl, p.tw4M, p.M);
     const ItemDesc &it = p.items[f.item];
     const uint32_t *X = op ? it.B : it.A;
     const int XL = (int)(op ? it.BL : it.AL);
@@ -225,16 +234,19 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(C
     }
   };
   unsigned u = blockIdx.x;
-  if (u < total) stage_copy(u);
+  if (u < total) stage_copy(u, 0);
   cp_async_commit();
-  for (; u < total; u += gridDim.x) {
-    const FwdUnit f = fwd_unit(p, u, nA, fd_tile, (unsigned)tiles);
+  // while the first unit's words cross: the tables and this thread's factors
+  tw16_build<L, NT>(twS, p.twL1);
+  table_to_smem<L, NT>(pwS, p.pw_fwd);
+  const ColTw16 ct = col_tw16<R>(s, t, p.tw4M, p.M);
+  for (int par = 0; u < total; u += gridDim.x, par ^= 1) {
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
     const int tl = (int)f.rest, op = f.op;
     const ItemDesc &it = p.items[f.item];
     const int col = tl * W + s;
     cp_async_wait<0>();
-    __syncthreads();  // the stage (every thread's copies) has landed; the last unit's factors are read
-    tile_tw16<R, W, NT>(fac, tl, twoM);  // read after block16's barriers
+    __syncthreads();  // the stage (every thread's copies) has landed
     const unsigned nd = (unsigned)(op ? it.ndB : it.ndA);  // below 2^30
     double2 *gbuf = op ? it.bufB : it.bufA;
     const int b = it.b;
@@ -270,10 +282,10 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(C
     }
     __syncthreads();  // every thread has cut its digits: the stage is free
     const unsigned un = u + gridDim.x;
-    if (un < total) stage_copy(un);
+    if (un < total) stage_copy(un, par ^ 1);
     cp_async_commit();
     block16<L, W, false>(v, t, s, tile, twS);
-    const OuterRun16 tw = outer_run16(fac, ct, t);
+    const OuterRun16 tw = outer_run16(fac + par * TILE_TW_N, ct, t);
     double2 w = tw.b0;
 #pragma unroll
     for (int i = 0; i < P16; i++) {
@@ -297,21 +309,22 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB)
   double2 *const buf0 = align1024(smraw);  // stage st's tile at buf0 + st * L * W
   double2 *twS = buf0 + 2 * L * W;
   double2 *pwS = twS + L;
-  double2 *fac = pwS + L;  // tile factors of unit parity st at fac + st * TILE_TW
-  tw16_build<L>(twS, p.twL1);
-  table_to_smem(pwS, p.pw_inv, L);
+  double2 *fac = pwS + L;  // tile factors of unit parity st at fac + st * TILE_TW_N
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
-  const unsigned tiles = p.S1 / W;
+  const FastDiv fd_tiles = p.fd_outer;
+  const unsigned tiles = fd_tiles.d;
   const unsigned total = (unsigned)p.nitems * tiles;  // far below 2^32
-  const FastDiv fd_tiles(tiles);
-  const double twoM = 2.0 * (double)p.M;
-  const ColTw16 ct = col_tw16<R>(s, t, twoM);
-  if (blockIdx.x < total) tile_tw16<R, W, NT>(fac, (int)(blockIdx.x % tiles), twoM);
+  if (blockIdx.x < total) tile_tw16<R, W>(fac, (int)(blockIdx.x - fd_tiles.div(blockIdx.x) * tiles), p.tw4M, p.M);
+  cp_async_commit();
+  tw16_build<L, NT>(twS, p.twL1);
+  table_to_smem<L, NT>(pwS, p.pw_inv);
+  const ColTw16 ct = col_tw16<R>(s, t, p.tw4M, p.M);
   if (tid == 0) {
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
     fence_mbar_init();
   }
+  cp_async_wait<0>();
   __syncthreads();
   pdl_wait();
   pdl_trigger();
@@ -347,7 +360,7 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB)
     double2 *bf = buf0 + st * L * W;
     double2 v[P16];
     {
-      const OuterRun16 tw = outer_run16(fac + st * TILE_TW, ct, t);
+      const OuterRun16 tw = outer_run16(fac + st * TILE_TW_N, ct, t);
       double2 w = tw.b0;
 #pragma unroll
       for (int i = 0; i < P16; i++) {
@@ -364,8 +377,9 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB)
       }
       return;
     }
-    // the next unit's tile factors (read after this unit's last barrier)
-    if (un < total) tile_tw16<R, W, NT>(fac + (st ^ 1) * TILE_TW, (int)(un % tiles), twoM);
+    // the next unit's tile factors (landed and published by this unit's last barriers)
+    if (un < total) tile_tw16<R, W>(fac + (st ^ 1) * TILE_TW_N, (int)(un - fd_tiles.div(un) * tiles), p.tw4M, p.M);
+    cp_async_commit();
     block16<L, W, true>(v, t, s, bf, twS);
 #pragma unroll
     for (int i = 0; i < P16; i++) {
@@ -375,6 +389,7 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB)
       err_acc = fmax(err_acc, round_check(z, re, im));
       bf[bidx<L>(n1, s)] = make_double2(re, im);
     }
+    cp_async_wait<0>();
     __syncthreads();
     // run records: one 8-column group of one row per (thread, q); L*G rows x
     // groups over NT threads

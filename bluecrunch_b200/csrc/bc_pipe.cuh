@@ -47,12 +47,16 @@ template <int L> struct PassTile {
   static constexpr size_t SMEM_OUTER_INV = SMEM_MID + (size_t)L * 16;
 };
 
-// Copy n table entries from global to shared memory (all threads of the CTA;
-// the caller's next barrier publishes them).
-__device__ __forceinline__ void table_to_smem(double2 *dst, const double2 *__restrict__ src, int n) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(&src[i]);
+// Copy the L entries of a table from global to shared memory (all NT threads,
+// loads issued together; the caller's next barrier publishes them).
+template <int L, int NT>
+__device__ __forceinline__ void table_to_smem(double2 *dst, const double2 *__restrict__ src) {
+#pragma unroll
+  for (int q = 0; q < (L + NT - 1) / NT; q++) {
+    const int i = threadIdx.x + q * NT;
+    if (L % NT == 0 || i < L) dst[i] = __ldg(&src[i]);
+  }
 }
-
 __device__ __forceinline__ double2 *align1024(unsigned char *p) {
   return reinterpret_cast<double2 *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
@@ -101,9 +105,8 @@ __device__ __forceinline__ void outer_twiddles(const Tw2 &T, int col, int t, dou
   else twiddle_run(T, (uint64_t)col * (4 * t - 1), false, (uint64_t)col * 4 * TC, w);
 }
 
-// e^{-2 pi i m/(2 h)} for |m| < 2h: sincospi of m/h.  With h = 2M it is the
-// outer passes' e^{-2 pi i m/(4M)}; with h = S1/2 the middle passes'
-// e^{-2 pi i m/(L2 Lr)}.
+// e^{-2 pi i m/(2 h)} for |m| < 2h: sincospi of m/h.  With h = S1/2 it is the
+// middle passes' e^{-2 pi i m/(L2 Lr)}.
 __device__ __forceinline__ double2 t4m(long long m, double h) {
   double sn, cs;
   sincospi((double)m / h, &sn, &cs);
@@ -119,7 +122,9 @@ __device__ __forceinline__ double2 t4m(long long m, double h) {
 // T(s x)): the TC + 1 tile factors T(tile W t) (t < TC) and T(tile W TC) are
 // computed once per unit by a few lanes of each warp (sincospi) into shared
 // memory, the column factors T(s t) and T(s TC) stay in registers.  No
-// global twiddle loads remain on the unit's path.
+// global twiddle loads remain on the unit's path: these passes run at 0.8 of
+// the memory's rate, and copying the factors' table entries ahead as the outer
+// passes do made them slower (forward 0.405 -> 0.430 ms at 2^25 points).
 template <int TC, int W, int NT>
 __device__ __forceinline__ void mid_tile_tw(double2 *fac, int tile, double h) {
   constexpr int NF = TC + 1, NW = NT / 32, PER = (NF + NW - 1) / NW;
@@ -137,18 +142,18 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB)
   double2 *const buf0 = align1024(smraw);  // stage st's tile at buf0 + st * L * W
   double2 *twS = buf0 + 2 * L * W;
   double2 *fac = twS + T::TWN;  // tile factors of unit parity st at fac + st * (TC + 1)
-  table_to_smem(twS, p.twL2, T::TWN);
+  table_to_smem<T::TWN, NT>(twS, p.twL2);
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
   const double h = 0.5 * (double)p.S1;
   const double2 cb = t4m((long long)s * t, h), cs = t4m((long long)s * TC, h);
   // unit counts stay far below 2^32 (a class holds at most 2^33 points, 2048 per unit)
-  const unsigned tiles = p.Lr / W;
+  const FastDiv fd_op = p.fd_op, fd_tile = p.fd_mid;
+  const unsigned tiles = fd_tile.d;
   // forward: the A units of every item, then the B slab's slots (map mB's
   // last coordinate is the slot); inverse: A only
-  const unsigned per_op = (unsigned)p.L1 * tiles;
+  const unsigned per_op = fd_op.d;
   const unsigned nA = INV ? (unsigned)p.nitems * per_op : fwd_units_a(p, per_op);
   const unsigned total = nA + (INV ? 0u : fwd_units_b(p, per_op));
-  const FastDiv fd_op(per_op), fd_tile(tiles);
   auto decode = [&](unsigned u, int &item, int &op, int &slot, int &blk, int &tile) {
     const FwdUnit f = fwd_unit(p, u, nA, fd_op, per_op);
     item = f.item;
@@ -243,12 +248,12 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_i
   double2 *const buf0 = align1024(smraw);  // stage st's tile at buf0 + st * L * W
   double2 *twS = buf0 + 2 * L * W;
   double2 *pwS = twS + T::TWN;
-  table_to_smem(twS, p.twL1, T::TWN);
-  table_to_smem(pwS, p.pw_inv, L);
+  table_to_smem<T::TWN, T::NT>(twS, p.twL1);
+  table_to_smem<L, T::NT>(pwS, p.pw_inv);
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
-  const unsigned tiles = p.S1 / W;
+  const FastDiv fd_tiles = p.fd_outer;
+  const unsigned tiles = fd_tiles.d;
   const unsigned total = (unsigned)p.nitems * tiles;  // far below 2^32
-  const FastDiv fd_tiles(tiles);
   if (tid == 0) {
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
@@ -384,8 +389,6 @@ __device__ __forceinline__ void rows_load(double2 *dst, const CUtensorMap *map, 
 template <int L, bool SQ>
 __global__ void __launch_bounds__(RowTile<L>::NT, RowTile<L>::MINB)
     k2_rows(ClassParams p, const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB) {
-  pdl_wait();
-  pdl_trigger();
   using R = RowTile<L>;
   constexpr int TC = L / PTS, NR = R::NR, NS = R::SLOTS;
   extern __shared__ unsigned char smraw[];
@@ -394,9 +397,9 @@ __global__ void __launch_bounds__(RowTile<L>::NT, RowTile<L>::MINB)
   double2 *twS = bufA0 + 2 * NS * NR * L;
   staged_tw_build<L>(twS, p.twLr);
   const int tid = threadIdx.x, rl = tid / TC, t = tid % TC;
-  const unsigned rows_item = p.M / L;
+  const FastDiv fd_rows = p.fd_rows;
+  const unsigned rows_item = fd_rows.d;
   const unsigned total = (unsigned)p.nitems * rows_item / NR;  // far below 2^32
-  const FastDiv fd_rows(rows_item);
   // row of the B slab for class row `row` (item i's B transform sits in its slot)
   auto brow = [&](unsigned row) -> unsigned {
     const unsigned item = fd_rows.div(row);
@@ -408,6 +411,8 @@ __global__ void __launch_bounds__(RowTile<L>::NT, RowTile<L>::MINB)
     fence_mbar_init();
   }
   __syncthreads();
+  pdl_wait();
+  pdl_trigger();
   unsigned u = blockIdx.x;
   unsigned pend = 0;  // bit k: a copy issued on bars[k] that has not been seen to land
 #pragma unroll
@@ -534,13 +539,10 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
   uint32_t *stg = reinterpret_cast<uint32_t *>(tile + L * W);  // 2 stages of STAGE_WORDS
   double2 *twS = reinterpret_cast<double2 *>(stg + 2 * K::STAGE_WORDS);
   double2 *pwS = twS + tw_entries<L>();
-  table_to_smem(twS, p.twL1, tw_entries<L>());
-  table_to_smem(pwS, p.pw_fwd, L);
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
-  const int tiles = p.S1 / W;
+  const int tiles = (int)p.fd_outer.d;
   const unsigned nA = fwd_units_a(p, (unsigned)tiles);
   const unsigned total = nA + fwd_units_b(p, (unsigned)tiles);  // far below 2^32
-  const FastDiv fd_tile((unsigned)tiles);
   // Row segment (n1, part) of tile tl starts one word below the word of digit
   // j0 = n1*S1 + tl*W + part*M.  S1 and M are multiples of 128, so that word is
   // n1*(S1 b/32) + part*(M b/32) + (tl*W*b >> 5), with the first two terms
@@ -551,7 +553,7 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
     return al16 ? (int)((((long long)tl * W * b >> 5) - 1) & 3) : 0;
   };
   auto stage_copy = [&](unsigned u, int st) {
-    const FwdUnit f = fwd_unit(p, u, nA, fd_tile, (unsigned)tiles);
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
     const int tl = (int)f.rest, op = f.op;
     const ItemDesc &it = p.items[f.item];
     const uint32_t *X = op ? it.B : it.A;
@@ -590,13 +592,16 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
   int st = 0;
   if (u < total) stage_copy(u, 0);
   cp_async_commit();
+  // while the first unit's words cross
+  table_to_smem<tw_entries<L>(), NT>(twS, p.twL1);
+  table_to_smem<L, NT>(pwS, p.pw_fwd);
   for (; u < total; u += gridDim.x) {
     const unsigned un = u + gridDim.x;
     if (un < total) stage_copy(un, st ^ 1);
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
-    const FwdUnit f = fwd_unit(p, u, nA, fd_tile, (unsigned)tiles);
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
     const int tl = (int)f.rest, op = f.op;
     const ItemDesc &it = p.items[f.item];
     const unsigned nd = (unsigned)(op ? it.ndB : it.ndA);  // below 2^30

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(32 * R5_WARPS, 2)
   pdl_trigger();
   const unsigned rows_item = p.M / R5_L;
   const unsigned total = (unsigned)p.nitems * rows_item;  // rows of the class, far below 2^32
-  const FastDiv fd_rows(rows_item);
+  const FastDiv fd_rows = p.fd_rows;
   const unsigned stride = gridDim.x * R5_WARPS;
   // row q of item i; B's rows sit in the item's B slot
   auto row_base = [&](unsigned row, bool opB) -> double2 * {

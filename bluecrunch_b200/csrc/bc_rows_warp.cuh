@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(32 * RW_WARPS, 2)
   pdl_trigger();
   const unsigned rows_item = p.M / RW_L;
   const unsigned total = (unsigned)p.nitems * rows_item;  // rows of the class, far below 2^32
-  const FastDiv fd_rows(rows_item);
+  const FastDiv fd_rows = p.fd_rows;
   const unsigned stride = gridDim.x * RW_WARPS;
   auto row_base = [&](unsigned row, bool opB) -> double2 * {
     const unsigned item = fd_rows.div(row);
