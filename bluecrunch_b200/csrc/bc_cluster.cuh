@@ -87,7 +87,7 @@ __device__ __forceinline__ void stage_limbs(uint32_t *dst, const uint32_t *__res
 
 template <int M, bool SQ>
 __global__ void __cluster_dims__(ClusterShape<M>::NC, 1, 1) __launch_bounds__(ClusterShape<M>::NT, 1)
-    k_cluster(ClassParams p) {
+    k_cluster(const __grid_constant__ ClassParams p) {
   namespace cg = cooperative_groups;
   using T = ClusterShape<M>;
   constexpr int NC = T::NC, S = T::S, P = T::P, TC = T::TC, NT = T::NT, NF = T::NF;
@@ -111,8 +111,12 @@ __global__ void __cluster_dims__(ClusterShape<M>::NC, 1, 1) __launch_bounds__(Cl
   double2 *const Y = rows + S;
   const int nclus = gridDim.x / NC;
   bool tables = false;
+  if (c == 0) {  // before the cluster's first barrier; nothing here is used before it
+    if (p.single)
+      for (unsigned i = tid; i < p.zero_n; i += NT) p.zero[i] = make_uint4(0, 0, 0, 0);
+  }
   for (int item = blockIdx.x / NC; item < p.nitems; item += nclus) {
-    const ItemDesc &it = p.items[item];
+    const ItemDesc &it = p.single ? p.one : p.items[item];
     const int AL = (int)it.AL, BL = (int)it.BL, b = it.b;
     uint32_t *const limbA = limb + 3, *const limbB = limbA + ((AL + 3 + 3) & ~3);
     stage_limbs(limbA, it.A, AL);
@@ -284,10 +288,16 @@ __global__ void __cluster_dims__(ClusterShape<M>::NC, 1, 1) __launch_bounds__(Cl
       U192 hn = {{rec[q * SLOTS + rr + 2].h0 + (unsigned long long)(me.c + dout), 0, 0}};
       const unsigned long long r = (unsigned long long)((q * S + c * P) / 8 + rr);
       write_run_words(it.C, it.nwords, r, nbits, h, hn);
-      if (q == SEG - 1 && c == NC - 1 && rr == RUNS - 1 && me.c + dout != 0) atomicOr(it.flags, FLAG_TOPCARRY);
+      if (q == SEG - 1 && c == NC - 1 && rr == RUNS - 1 && me.c + dout != 0) {
+        atomicOr(it.flags, FLAG_TOPCARRY);
+        __threadfence();
+      }
     }
     for (unsigned long long w = it.nwords + (unsigned)(c * NT + tid); w < it.CL; w += NC * NT) it.C[w] = 0;
     __syncthreads();  // the limbs, runs and maps are free for the next product
+    // the errors were published before the second cluster barrier, the flag of
+    // a carry out of the product by this CTA
+    if (tid == 0 && c == NC - 1) publish_outcome(it);
     // ---- end
   }
 }

@@ -1303,7 +1303,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   }
   const size_t off_status = off; off += align256(status_words * 4);
   const size_t zero_end = off;
-  const size_t off_desc = off; off += align256(nw * sizeof(ItemDesc));
+  const size_t off_desc = off; off += align256(nw * sizeof(ItemDesc));  // right after the zeroed region
   // B-slot owners of every class, after the descriptors (copied with them)
   std::map<std::pair<size_t, bool>, size_t> own_off;
   size_t own_words = 0;
@@ -1366,7 +1366,6 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     if (pin_out_off[i] != SIZE_MAX) runs[i].dC = (uint32_t *)(base + off_stage_out + pin_out_off[i]);
     else runs[i].dC = (runs[i].hostC || runs[i].stagedC) ? (uint32_t *)(base + slots[i].off_dC) : d.C;
   }
-  CK(cudaMemsetAsync(base + off_err, 0, zero_end - off_err, g.stream));
 
   // ---- descriptors
   std::vector<ItemDesc> desc(nw);
@@ -1401,6 +1400,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
       tile0 += pl.ntiles;
       it.err = (unsigned long long *)(base + off_err) + i;
       it.flags = (unsigned int *)(base + off_flags) + i;
+      it.outcome = nullptr;  // set when the pinned block is there
       it.b = pl.b;
       it.square = pl.square ? 1 : 0;
       it.a16 = stage16_ok(it.A, pl);
@@ -1409,21 +1409,37 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     }
   }
   ItemDesc *ddesc = (ItemDesc *)(base + off_desc);
-  // descriptors and, later, the outcomes go through one pinned block: the
-  // descriptors at its start, the outcomes (err, flags) after them
-  // (the B-slot owners right after the descriptors, as in the arena)
+  // One pinned block holds the zeros, the descriptors and the B-slot owners
+  // as they lie in the arena (one copy), and after them the outcomes, which
+  // each item's last kernel writes there.  A product alone in its call needs
+  // no copy: its descriptor goes with its first kernel's parameters, and that
+  // kernel clears the region (ClassParams::single).  Zeros above kZeroCopy
+  // bytes (the status words of very long products) are a memset of their own.
+  const bool single = nw == 1 && !graph;
+  constexpr size_t kZeroCopy = size_t(64) << 10;
+  const size_t zero_bytes = zero_end - off_err, zero_copy = zero_bytes <= kZeroCopy ? zero_bytes : 0;
   const size_t desc_bytes = align256(nw * sizeof(ItemDesc)) + own_words * 4;
-  const size_t pin_desc = align256(desc_bytes), pin_outc = off_flags + nw * 4 - off_err;
-  if ((r = pin_small_reserve(pin_desc + pin_outc))) return r;
-  memcpy(g.pin_small, desc.data(), nw * sizeof(ItemDesc));
-  {
-    int *po = (int *)((char *)g.pin_small + align256(nw * sizeof(ItemDesc)));
+  const size_t pin_outc = align256(zero_copy + desc_bytes);
+  if ((r = pin_small_reserve(pin_outc + nw * 16))) return r;
+  unsigned long long *outc = (unsigned long long *)((char *)g.pin_small + pin_outc);
+  for (size_t k = 0; k < nw; k++) {
+    desc[k].outcome = outc + 2 * order[k];
+    // unless a kernel says otherwise: nothing ran
+    outc[2 * k] = 0x7ff0000000000000ull;  // +infinity
+    outc[2 * k + 1] = FLAG_TIMEOUT;
+  }
+  if (!single) {
+    char *pin = (char *)g.pin_small;
+    memset(pin, 0, zero_copy);
+    memcpy(pin + zero_copy, desc.data(), nw * sizeof(ItemDesc));
+    int *po = (int *)(pin + zero_copy + align256(nw * sizeof(ItemDesc)));
     for (auto &c : classes) {
       const std::vector<int> &own = owners[c.first];
       std::copy(own.begin(), own.end(), po + own_off[c.first]);
     }
+    if (!zero_copy) CK(cudaMemsetAsync(base + off_err, 0, zero_bytes, g.stream));
+    CK(cudaMemcpyAsync((char *)ddesc - zero_copy, pin, zero_copy + desc_bytes, cudaMemcpyHostToDevice, g.stream));
   }
-  CK(cudaMemcpyAsync(ddesc, g.pin_small, desc_bytes, cudaMemcpyHostToDevice, g.stream));
   const int *down = (const int *)((const char *)ddesc + align256(nw * sizeof(ItemDesc)));
   unsigned int *ctr = (unsigned int *)(base + off_ctr);
 
@@ -1477,9 +1493,15 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     p.slabA = (double2 *)(base + slab[c.first].offA);
     p.slabB = sq ? nullptr : (double2 *)(base + slab[c.first].offB);
     p.nb = sq ? 0 : (int)owners[c.first].size();
-    p.bowner = sq ? nullptr : down + own_off[c.first];
+    p.bowner = sq || single ? nullptr : down + own_off[c.first];
     p.fwd_ops = 0;
     p.slab_elems = align256(s.M * 16) / 16;
+    p.single = single ? 1 : 0;
+    if (single) {
+      p.one = desc[0];
+      p.zero = (uint4 *)(base + off_err);
+      p.zero_n = (unsigned)(zero_bytes / 16);
+    }
     unsigned long long tiles = 0;
     bool w16 = true;  // every item of the class has width 16: the carry pass specialised for it
     for (size_t k = first; k < first + n; k++) {
@@ -1510,15 +1532,23 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   CK(cudaEventRecord(g.ev1, g.stream));
   st->classes += classes.size();
 
+  // ---- outputs that fit one chunk of the ring start on their way before the
+  // outcomes are known (they are kept only if the product passed)
+  const bool early_out = stage_out && stage_out <= kRingChunk;
+  if (early_out) {
+    if ((r = ring_ready())) return r;
+    CK(cudaMemcpyAsync(g_ring.half[1], base + off_stage_out, stage_out, cudaMemcpyDeviceToHost, g.stream));
+  }
+
   // ---- outcomes, then outputs of the products that passed
-  char *outc = (char *)g.pin_small + pin_desc;
-  CK(cudaMemcpyAsync(outc, base + off_err, pin_outc, cudaMemcpyDeviceToHost, g.stream));
   pt.next(&g_prof.wait);
   CK(cudaStreamSynchronize(g.stream));
   std::vector<unsigned long long> errs(nw);
   std::vector<unsigned> flags(nw);
-  memcpy(errs.data(), outc, nw * 8);
-  memcpy(flags.data(), outc + (off_flags - off_err), nw * 4);
+  for (size_t i = 0; i < nw; i++) {
+    errs[i] = outc[2 * i];
+    flags[i] = (unsigned)outc[2 * i + 1];
+  }
   pt.next(&g_prof.copy_out);
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, g.ev0, g.ev1));
@@ -1563,7 +1593,14 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     for (size_t i = 0; i < nw; i++)
       if (ok[i] && pin_out_off[i] != SIZE_MAX)
         jobs.push_back({pin_out_off[i], (char *)items[works[i]->idx].C, items[works[i]->idx].CL * 4});
-    if ((r = stage_d2h(base + off_stage_out, jobs, stage_out))) return r;
+    if (early_out) {
+      std::vector<CopyJob> pieces;
+      size_t j = 0;
+      window_pieces(jobs, j, 0, stage_out, g_ring.half[1], false, pieces);
+      par_copy(pieces);
+    } else if ((r = stage_d2h(base + off_stage_out, jobs, stage_out))) {
+      return r;
+    }
     st->d2h_bytes += stage_out;
     g_prof.bytes_out += stage_out;
   }

@@ -56,6 +56,7 @@ struct ItemDesc {
   int b;
   int square;
   int a16, b16;                   // operand A / B starts on a 16-byte boundary
+  unsigned long long *outcome;    // two words of pinned host memory: err and flags, written by the item's last kernel
   int bslot;                      // slot of B's transform in the class's B slab (shared by items with the same B)
 };
 
@@ -90,7 +91,67 @@ struct ClassParams {
   FastDiv fd_outer, fd_op, fd_mid, fd_rows;
   double2 *slabA, *slabB;          // the class's A and B slabs (item i at slab + i*slab_elems)
   unsigned long long slab_elems;
+  // A product alone in its call: its descriptor comes with the first kernel's
+  // parameters (single = 1) and that kernel stores it to items[0] for the
+  // others and clears the zero_n 16-byte words at `zero` (errors, flags,
+  // counters, lookback status), instead of a copy and a memset before it.
+  int single;
+  unsigned zero_n;
+  uint4 *zero;
+  ItemDesc one;
 };
+
+// What the outer forward pass reads of an item's operand, by value: from the
+// parameters' constant bank for a product alone in its call.
+struct FwdOperand {
+  const uint32_t *X;
+  double2 *buf;
+  int XL, b;
+  unsigned nd;  // below 2^30
+  bool al16;
+};
+__device__ __forceinline__ FwdOperand fwd_operand(const ClassParams &p, int item, int op) {
+  FwdOperand o;
+  if (p.single) {
+    o.X = op ? p.one.B : p.one.A;
+    o.buf = op ? p.one.bufB : p.one.bufA;
+    o.XL = (int)(op ? p.one.BL : p.one.AL);
+    o.nd = (unsigned)(op ? p.one.ndB : p.one.ndA);
+    o.b = p.one.b;
+    o.al16 = op ? p.one.b16 : p.one.a16;
+  } else {
+    const ItemDesc &it = p.items[item];
+    o.X = op ? it.B : it.A;
+    o.buf = op ? it.bufB : it.bufA;
+    o.XL = (int)(op ? it.BL : it.AL);
+    o.nd = (unsigned)(op ? it.ndB : it.ndA);
+    o.b = it.b;
+    o.al16 = op ? it.b16 : it.a16;
+  }
+  return o;
+}
+
+// The first kernel's part for a product alone in its call (see ClassParams);
+// what the call's later kernels read is complete when this one has ended.
+__device__ __forceinline__ void first_kernel_setup(const ClassParams &p) {
+  if (!p.single) return;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < p.zero_n; i += gridDim.x * blockDim.x)
+    p.zero[i] = make_uint4(0, 0, 0, 0);
+  constexpr unsigned N = sizeof(ItemDesc) / 8;
+  static_assert(sizeof(ItemDesc) % 8 == 0, "copied by 8-byte words");
+  if (blockIdx.x == 0)
+    for (unsigned i = threadIdx.x; i < N; i += blockDim.x)
+      reinterpret_cast<unsigned long long *>(const_cast<ItemDesc *>(p.items))[i] =
+          reinterpret_cast<const unsigned long long *>(&p.one)[i];
+}
+
+// An item's outcome to the host (a posted write of two words), when all that
+// sets its error and flags is done and visible.
+__device__ __forceinline__ void publish_outcome(const ItemDesc &it) {
+  if (!it.outcome) return;
+  it.outcome[0] = *reinterpret_cast<volatile const unsigned long long *>(it.err);
+  it.outcome[1] = *reinterpret_cast<volatile const unsigned *>(it.flags);
+}
 
 // One unit of a forward pass: operand `op` of item `item` (for B, the owner
 // of slot `slot`), and the unit's index `rest` inside that operand's
@@ -369,7 +430,7 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
   __shared__ uint32_t lastf[CARRY_RPT * NW];   // map of each warp's last run
   __shared__ uint8_t fm[CARRY_TILE_RUNS];      // all maps, then the carries + 1 (only when the tile is scanned)
   __shared__ uint32_t sw[65];
-  __shared__ unsigned s_unit[2];
+  __shared__ unsigned s_unit[2], s_last;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (tid == 0) s_unit[0] = atomicAdd(p.counter, 1u);
   pdl_wait();
@@ -536,6 +597,15 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
     }
     __syncthreads();
   }
+  // the last CTA to finish tells the host how the class's items went
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(p.counter + 1, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (s_last)
+    for (int i = tid; i < p.nitems; i += CARRY_NT) publish_outcome(p.items[i]);
 }
 
 // ------------------------------------------------------------------ small
@@ -623,7 +693,9 @@ __global__ void __launch_bounds__(M / PTS, 1) k_small(ClassParams p) {
     write_run_words(it.C, it.nwords, (unsigned long long)(NR + t), nbits, him, nim);
     if (t == TC - 1 && rim.c + dout_im != 0) atomicOr(it.flags, FLAG_TOPCARRY);
     for (unsigned long long w = it.nwords + t; w < it.CL; w += TC) it.C[w] = 0;
+    __threadfence();  // the warps' error and flag updates, before thread 0 reads them
     __syncthreads();
+    if (t == 0) publish_outcome(it);
   }
 }
 

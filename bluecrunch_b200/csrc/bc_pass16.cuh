@@ -176,7 +176,7 @@ __device__ __forceinline__ OuterRun16 outer_run16(const double2 *fac, const ColT
 // next unit's words are copied (cp.async) as soon as this unit's digits are
 // cut, and land while this unit is transformed and stored.
 template <int L>
-__global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(ClassParams p) {
+__global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(const __grid_constant__ ClassParams p) {
   pdl_trigger();  // the first pass of a class: launched normally, lets the next one start early
   using T = Pass16<L>;
   using K = PackTile<L>;
@@ -201,16 +201,16 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(C
   // still at the unit before read the other set)
   auto stage_copy = [&](unsigned u, int par) {
     const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
-    const int tl = (int)f.rest, op = f.op;
+    const int tl = (int)f.rest;
     tile_tw16<R, W>(fac + par * TILE_TW_N, tl, p.tw4M, p.M);
-    const ItemDesc &it = p.items[f.item];
-    const uint32_t *X = op ? it.B : it.A;
-    const int XL = (int)(op ? it.BL : it.AL);
+    const FwdOperand it = fwd_operand(p, f.item, f.op);
+    const uint32_t *X = it.X;
+    const int XL = it.XL;
     const int b = it.b;
-    const bool al16 = op ? it.b16 : it.a16;
+    const bool al16 = it.al16;
     const int RW = (int)((unsigned)p.S1 * (unsigned)b / 32), PW = (int)((unsigned)p.M * (unsigned)b / 32);
     const int wbase = ((tl * W * b) >> 5) - 1 - seg_shift(tl, b, al16);
-    const int parts = (op ? it.ndB : it.ndA) > (unsigned long long)p.M ? 2 : 1;
+    const int parts = it.nd > (unsigned)p.M ? 2 : 1;
     if (al16) {
       constexpr int CH = K::SEGW4 / 4;
       const int NCH = parts * L * CH;
@@ -236,21 +236,22 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(C
   unsigned u = blockIdx.x;
   if (u < total) stage_copy(u, 0);
   cp_async_commit();
+  first_kernel_setup(p);
   // while the first unit's words cross: the tables and this thread's factors
   tw16_build<L, NT>(twS, p.twL1);
   table_to_smem<L, NT>(pwS, p.pw_fwd);
   const ColTw16 ct = col_tw16<R>(s, t, p.tw4M, p.M);
   for (int par = 0; u < total; u += gridDim.x, par ^= 1) {
     const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
-    const int tl = (int)f.rest, op = f.op;
-    const ItemDesc &it = p.items[f.item];
+    const int tl = (int)f.rest;
+    const FwdOperand it = fwd_operand(p, f.item, f.op);
     const int col = tl * W + s;
     cp_async_wait<0>();
     __syncthreads();  // the stage (every thread's copies) has landed
-    const unsigned nd = (unsigned)(op ? it.ndB : it.ndA);  // below 2^30
-    double2 *gbuf = op ? it.bufB : it.bufA;
+    const unsigned nd = it.nd;
+    double2 *gbuf = it.buf;
     const int b = it.b;
-    const bool al16 = op ? it.b16 : it.a16;
+    const bool al16 = it.al16;
     const unsigned rel = 32u * (1u + (unsigned)seg_shift(tl, b, al16)) + (unsigned)((tl * W * b) & 31) +
                          (unsigned)(s * b);  // bit of digit j0+s in its staged segment
     const unsigned wi = (rel - 1) >> 5, sh = (rel - 1) & 31;

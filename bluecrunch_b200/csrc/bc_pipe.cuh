@@ -529,7 +529,7 @@ template <int L> struct PackTile {
 };
 
 template <int L>
-__global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_fwd(ClassParams p) {
+__global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_fwd(const __grid_constant__ ClassParams p) {
   pdl_trigger();  // the first pass of a class: launched normally, lets the next one start early
   using T = PassTile<L>;
   using K = PackTile<L>;
@@ -554,18 +554,18 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
   };
   auto stage_copy = [&](unsigned u, int st) {
     const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
-    const int tl = (int)f.rest, op = f.op;
-    const ItemDesc &it = p.items[f.item];
-    const uint32_t *X = op ? it.B : it.A;
+    const int tl = (int)f.rest;
+    const FwdOperand it = fwd_operand(p, f.item, f.op);
+    const uint32_t *X = it.X;
     // word indices fit an int: operands and transforms stay below 2^29 words
-    const int XL = (int)(op ? it.BL : it.AL);
+    const int XL = it.XL;
     const int b = it.b;
-    const bool al16 = op ? it.b16 : it.a16;
+    const bool al16 = it.al16;
     const int RW = (int)((unsigned)p.S1 * (unsigned)b / 32), PW = (int)((unsigned)p.M * (unsigned)b / 32);
     const int wbase = ((tl * W * b) >> 5) - 1 - seg_shift(tl, b, al16);
     uint32_t *dst = stg + st * K::STAGE_WORDS;
     // the imaginary parts hold digits M and up: none when nd <= M
-    const int parts = (op ? it.ndB : it.ndA) > (unsigned long long)p.M ? 2 : 1;
+    const int parts = it.nd > (unsigned)p.M ? 2 : 1;
     if (al16) {
       constexpr int CH = K::SEGW4 / 4;
       const int NCH = parts * L * CH;
@@ -592,6 +592,7 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
   int st = 0;
   if (u < total) stage_copy(u, 0);
   cp_async_commit();
+  first_kernel_setup(p);
   // while the first unit's words cross
   table_to_smem<tw_entries<L>(), NT>(twS, p.twL1);
   table_to_smem<L, NT>(pwS, p.pw_fwd);
@@ -602,14 +603,14 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
     cp_async_wait<1>();
     __syncthreads();
     const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
-    const int tl = (int)f.rest, op = f.op;
-    const ItemDesc &it = p.items[f.item];
-    const unsigned nd = (unsigned)(op ? it.ndB : it.ndA);  // below 2^30
-    double2 *gbuf = op ? it.bufB : it.bufA;
+    const int tl = (int)f.rest;
+    const FwdOperand it = fwd_operand(p, f.item, f.op);
+    const unsigned nd = it.nd;
+    double2 *gbuf = it.buf;
     const int b = it.b;
     const uint32_t *seg = stg + st * K::STAGE_WORDS;
     const int col = tl * W + s;
-    const bool al16 = op ? it.b16 : it.a16;
+    const bool al16 = it.al16;
     const unsigned rel = 32u * (1u + (unsigned)seg_shift(tl, b, al16)) + (unsigned)((tl * W * b) & 31) +
                          (unsigned)(s * b);  // bit of digit j0+s in its staged segment
     const unsigned wi = (rel - 1) >> 5, sh = (rel - 1) & 31;
