@@ -1420,13 +1420,14 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   const size_t zero_bytes = zero_end - off_err, zero_copy = zero_bytes <= kZeroCopy ? zero_bytes : 0;
   const size_t desc_bytes = align256(nw * sizeof(ItemDesc)) + own_words * 4;
   const size_t pin_outc = align256(zero_copy + desc_bytes);
-  if ((r = pin_small_reserve(pin_outc + nw * 16))) return r;
+  if ((r = pin_small_reserve(pin_outc + nw * 24))) return r;
   unsigned long long *outc = (unsigned long long *)((char *)g.pin_small + pin_outc);
   for (size_t k = 0; k < nw; k++) {
-    desc[k].outcome = outc + 2 * order[k];
+    desc[k].outcome = outc + 3 * order[k];
     // unless a kernel says otherwise: nothing ran
-    outc[2 * k] = 0x7ff0000000000000ull;  // +infinity
-    outc[2 * k + 1] = FLAG_TIMEOUT;
+    outc[3 * k] = 0x7ff0000000000000ull;  // +infinity
+    outc[3 * k + 1] = FLAG_TIMEOUT;
+    outc[3 * k + 2] = 0;
   }
   if (!single) {
     char *pin = (char *)g.pin_small;
@@ -1546,8 +1547,8 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   std::vector<unsigned long long> errs(nw);
   std::vector<unsigned> flags(nw);
   for (size_t i = 0; i < nw; i++) {
-    errs[i] = outc[2 * i];
-    flags[i] = (unsigned)outc[2 * i + 1];
+    errs[i] = outc[3 * i];
+    flags[i] = (unsigned)(outc[3 * i + 1] | outc[3 * i + 2]);
   }
   pt.next(&g_prof.copy_out);
   float ms = 0;

@@ -56,7 +56,7 @@ struct ItemDesc {
   int b;
   int square;
   int a16, b16;                   // operand A / B starts on a 16-byte boundary
-  unsigned long long *outcome;    // two words of pinned host memory: err and flags, written by the item's last kernel
+  unsigned long long *outcome;    // three words of pinned host memory: err, flags, and flags of a carry wait that gave up
   int bslot;                      // slot of B's transform in the class's B slab (shared by items with the same B)
 };
 
@@ -145,12 +145,15 @@ __device__ __forceinline__ void first_kernel_setup(const ClassParams &p) {
           reinterpret_cast<const unsigned long long *>(&p.one)[i];
 }
 
-// An item's outcome to the host (a posted write of two words), when all that
-// sets its error and flags is done and visible.
-__device__ __forceinline__ void publish_outcome(const ItemDesc &it) {
+// An item's outcome to the host (posted writes), once what sets its error and
+// flags is done and visible, by the thread that knows of a carry out of the
+// product.
+__device__ __forceinline__ void publish_outcome(const ItemDesc &it, unsigned more_flags = 0) {
   if (!it.outcome) return;
-  it.outcome[0] = *reinterpret_cast<volatile const unsigned long long *>(it.err);
-  it.outcome[1] = *reinterpret_cast<volatile const unsigned *>(it.flags);
+  const unsigned long long e = *reinterpret_cast<volatile const unsigned long long *>(it.err);
+  const unsigned f = *reinterpret_cast<volatile const unsigned *>(it.flags);
+  it.outcome[0] = e;
+  it.outcome[1] = f | more_flags;
 }
 
 // One unit of a forward pass: operand `op` of item `item` (for B, the owner
@@ -430,7 +433,7 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
   __shared__ uint32_t lastf[CARRY_RPT * NW];   // map of each warp's last run
   __shared__ uint8_t fm[CARRY_TILE_RUNS];      // all maps, then the carries + 1 (only when the tile is scanned)
   __shared__ uint32_t sw[65];
-  __shared__ unsigned s_unit[2], s_last;
+  __shared__ unsigned s_unit[2];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (tid == 0) s_unit[0] = atomicAdd(p.counter, 1u);
   pdl_wait();
@@ -516,7 +519,10 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
         if (!known) {
           bool timed_out = false;
           din = carry_lookback(it.status, tile, &timed_out);
-          if (timed_out) atomicOr(it.flags, FLAG_TIMEOUT);
+          if (timed_out) {
+            atomicOr(it.flags, FLAG_TIMEOUT);
+            if (it.outcome) it.outcome[2] = FLAG_TIMEOUT;
+          }
           if (!fixed) me.store(ST_INC | (uint32_t)(fn_apply(agg, din) + 1), cuda::memory_order_relaxed);
         }
         sw[0] = (uint32_t)(din + 1);
@@ -562,7 +568,14 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
             low[nr] = nr < CARRY_TILE_RUNS && r + 1 < nrec
                           ? (uint32_t)(rec[k + 1].h0 + (unsigned long long)(c[q] + dout)) : 0u;
           }
-          if (r + 1 == nrec && c[q] + dout != 0) atomicOr(it.flags, FLAG_TOPCARRY);
+          unsigned top = 0;
+          if (r + 1 == nrec && c[q] + dout != 0) {
+            top = FLAG_TOPCARRY;
+            atomicOr(it.flags, top);
+          }
+          // the item's last run: its error and the flags of the passes before
+          // are complete, so this thread tells the host
+          if (r + 1 == nruns) publish_outcome(it, top);
         }
       }
     }
@@ -597,15 +610,6 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
     }
     __syncthreads();
   }
-  // the last CTA to finish tells the host how the class's items went
-  if (tid == 0) {
-    __threadfence();
-    s_last = atomicAdd(p.counter + 1, 1u) == gridDim.x - 1;
-    __threadfence();
-  }
-  __syncthreads();
-  if (s_last)
-    for (int i = tid; i < p.nitems; i += CARRY_NT) publish_outcome(p.items[i]);
 }
 
 // ------------------------------------------------------------------ small
