@@ -1716,6 +1716,15 @@ struct DevBuf {
 };
 
 // ------------------------------------------------------------------ radix conversion leaves
+// `count` leaves whose descriptors are in device memory.
+int launch_radix_leaves(const RadixLeaf *leaves, size_t count, double alpha, unsigned *flag) {
+  const unsigned grid =
+      (unsigned)std::min<size_t>((count + RADIX_WARPS - 1) / RADIX_WARPS, (size_t)g.sm_count * 16);
+  k_radix_leaves<<<grid, 32 * RADIX_WARPS, 0, g.stream>>>(leaves, (int)count, alpha, flag);
+  CK(cudaGetLastError());
+  return BC_OK;
+}
+
 // Leaves whose fractions and digits are already in device memory, in one launch.
 int radix_leaves_device(const std::vector<RadixLeaf> &d, double alpha) {
   if (d.empty()) return BC_OK;
@@ -1725,11 +1734,7 @@ int radix_leaves_device(const std::vector<RadixLeaf> &d, double alpha) {
   char *base = g.arena;
   CK(cudaMemcpyAsync(base, d.data(), d.size() * sizeof(RadixLeaf), cudaMemcpyHostToDevice, g.stream));
   CK(cudaMemsetAsync(base + o_flag, 0, 256, g.stream));
-  const unsigned grid =
-      (unsigned)std::min<size_t>((d.size() + RADIX_WARPS - 1) / RADIX_WARPS, (size_t)g.sm_count * 16);
-  k_radix_leaves<<<grid, 32 * RADIX_WARPS, 0, g.stream>>>((const RadixLeaf *)base, (int)d.size(), alpha,
-                                                          (unsigned *)(base + o_flag));
-  CK(cudaGetLastError());
+  if ((r = launch_radix_leaves((const RadixLeaf *)base, d.size(), alpha, (unsigned *)(base + o_flag)))) return r;
   unsigned flag = 0;
   CK(cudaMemcpyAsync(&flag, base + o_flag, 4, cudaMemcpyDeviceToHost, g.stream));
   CK(cudaStreamSynchronize(g.stream));
@@ -1772,11 +1777,7 @@ int radix_leaves_locked(const bc_radix_leaf *lv, size_t count, double alpha) {
   if ((r = stage_h2d(base + o_in, jobs, in_bytes))) return r;
   CK(cudaMemcpyAsync(base + o_desc, d.data(), count * sizeof(RadixLeaf), cudaMemcpyHostToDevice, g.stream));
   CK(cudaMemsetAsync(base + o_flag, 0, 256, g.stream));
-  const unsigned grid =
-      (unsigned)std::min<size_t>((count + RADIX_WARPS - 1) / RADIX_WARPS, (size_t)g.sm_count * 16);
-  k_radix_leaves<<<grid, 32 * RADIX_WARPS, 0, g.stream>>>((const RadixLeaf *)(base + o_desc), (int)count, alpha,
-                                                          (unsigned *)(base + o_flag));
-  CK(cudaGetLastError());
+  if ((r = launch_radix_leaves((const RadixLeaf *)(base + o_desc), count, alpha, (unsigned *)(base + o_flag)))) return r;
   unsigned flag = 0;
   CK(cudaMemcpyAsync(&flag, base + o_flag, 4, cudaMemcpyDeviceToHost, g.stream));
   CK(cudaStreamSynchronize(g.stream));

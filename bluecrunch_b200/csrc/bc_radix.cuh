@@ -18,9 +18,22 @@
 // zero, is that same register.  Limbs above n are not held: carries only move
 // up, so they never reach limb n (in the first round the window reaches limb
 // len >= n, but what it computes above n is dropped with the carry out).
-// Each lane multiplies its limbs with a local carry chain; the carry out of a
-// lane enters the next lane's lowest limb, and a carry out of that limb
-// (astronomically rare) ripples further by a bounded loop.
+//
+// What bounds it: the instructions of one round after the other, some hundreds
+// of rounds, with about one warp per scheduler when leaves are few.  So no
+// round has a carry chain: limb q holds s_q < 2^33, its low word plus the high
+// word of the limb below, and the next round multiplies that (33 x 30 bits fit
+// 64); a lane's last limb keeps 32 bits and hands bit 32 on with its high
+// word.  Exact values are needed in two places only.  The digit: limb n plus
+// the carry out of limb n - 1, known from that limb's bit 32 unless its low
+// word is all ones (then, one round in 2^32, every carry is resolved).  And a
+// limb that the window's low end passes (at most one a round, alpha < 1; the
+// same register for every lane): nothing lies below it, so its bit 32 is the
+// carry that it hands to the next limb before it is cleared.  512 leaves of
+// 830 digits: 0.40 ms, 16,384 of them 4.8 ms; with a carry chain through every
+// limb and round 0.47 ms for the former at best, with the clearing by a mask
+// over the registers 0.56, on four warps each (eight limbs per lane, a barrier
+// per round) 0.41 and 8.2 ms.
 #pragma once
 #include <cstdint>
 
@@ -37,8 +50,39 @@ struct RadixLeaf {
   uint32_t len, n, k, pad;
 };
 
-__global__ void __launch_bounds__(32 * RADIX_WARPS) k_radix_leaves(const RadixLeaf *leaves, int count, double alpha,
-                                                                 unsigned *flags) {
+// All carries of a leaf's limbs: every s_q below 2^32 but lane 31's last one
+// (limb n).  Bounded: a carry passes at most 32 lanes.
+__device__ __forceinline__ void radix_resolve(unsigned long long (&s)[RS], int lane) {
+  unsigned long long c = 0;
+  for (int round = 0; round <= 32; round++) {
+#pragma unroll
+    for (int q = 0; q < RS; q++) {
+      s[q] += c;
+      c = 0;
+      if (q + 1 < RS || lane != 31) {
+        c = s[q] >> 32;
+        s[q] &= 0xffffffffull;
+      }
+    }
+    c = __shfl_up_sync(~0u, (uint32_t)c, 1);
+    if (lane == 0) c = 0;
+    if (!__any_sync(~0u, c != 0)) break;
+  }
+}
+
+// Limb q of a lane leaves the window: its carry to the limb above (a lane's
+// last limb has 32 bits), then zero.  By a switch over the registers: an index
+// would put them in local memory.
+template <int q>
+__device__ __forceinline__ void radix_drop(unsigned long long (&s)[RS], bool mine) {
+  if (mine) {
+    if constexpr (q + 1 < RS) s[q + 1] += s[q] >> 32;
+    s[q] = 0;
+  }
+}
+
+__global__ void __launch_bounds__(32 * RADIX_WARPS, 2) k_radix_leaves(const RadixLeaf *leaves, int count, double alpha,
+                                                                    unsigned *flags) {
   __shared__ uint32_t stage[RADIX_WARPS][RADIX_WINDOW + RADIX_WINDOW / 32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   uint32_t *sm = stage[wib];
@@ -59,55 +103,55 @@ __global__ void __launch_bounds__(32 * RADIX_WARPS) k_radix_leaves(const RadixLe
       sm[t + (t >> 5)] = (j >= 0 && j < (int)lf.len) ? lf.y[j] : 0u;
     }
     __syncwarp();
-    uint32_t x[RS];
+    unsigned long long x[RS];  // s_q
 #pragma unroll
     for (int q = 0; q < RS; q++) {
       const int t = lane * RS + q;
       x[q] = sm[t + (t >> 5)];
     }
     __syncwarp();
-    const int j0 = lane * RS + base;  // limb of x[0]
+    int lo = 0;    // low end of the round's window
+    int ends = 0;  // floor(alpha (i - 1)) of 32 rounds i, one per lane
     for (uint32_t i = 1; i <= lf.k; i++) {
-      const int lo = i == 1 ? 0 : (int)floor(alpha * (double)(i - 1));
-      // rounds after the first: the window's top limb (limb n, the last
-      // digit) enters as zero
-      if (i > 1 && lane == 31) x[RS - 1] = 0;
+      // limbs that have just left the window (limbs below base are not held)
+      if (((i - 1) & 31) == 0) ends = (int)floor(alpha * (double)((i - 1) + (uint32_t)lane));
+      const int lo_now = i == 1 ? 0 : __shfl_sync(~0u, ends, (int)((i - 1) & 31));
+      for (; lo < lo_now; lo++) {
+        const int g = lo - base;
+        const bool mine = lane == (g >> 5);
+        switch (g & 31) {
+#define RADIX_DROP(q) case q: radix_drop<q>(x, mine); break;
+          RADIX_DROP(0) RADIX_DROP(1) RADIX_DROP(2) RADIX_DROP(3) RADIX_DROP(4) RADIX_DROP(5) RADIX_DROP(6)
+          RADIX_DROP(7) RADIX_DROP(8) RADIX_DROP(9) RADIX_DROP(10) RADIX_DROP(11) RADIX_DROP(12) RADIX_DROP(13)
+          RADIX_DROP(14) RADIX_DROP(15) RADIX_DROP(16) RADIX_DROP(17) RADIX_DROP(18) RADIX_DROP(19) RADIX_DROP(20)
+          RADIX_DROP(21) RADIX_DROP(22) RADIX_DROP(23) RADIX_DROP(24) RADIX_DROP(25) RADIX_DROP(26) RADIX_DROP(27)
+          RADIX_DROP(28) RADIX_DROP(29) RADIX_DROP(30) RADIX_DROP(31)
+#undef RADIX_DROP
+        }
+      }
       // multiply the window [lo, n] by 10^9
-      uint32_t c = 0;
+      uint32_t h = 0;  // high word of the limb below
 #pragma unroll
       for (int q = 0; q < RS; q++) {
-        if (j0 + q >= lo) {
-          const unsigned long long v = (unsigned long long)x[q] * DEC_BASE + c;
-          x[q] = (uint32_t)v;
-          c = (uint32_t)(v >> 32);
-        }
+        const unsigned long long v = (unsigned long long)(uint32_t)x[q] * DEC_BASE;
+        const uint32_t hi = (uint32_t)(v >> 32) + (uint32_t)(x[q] >> 32) * DEC_BASE;
+        x[q] = (unsigned long long)(uint32_t)v + h;
+        h = hi;
       }
-      // the carry out of lane l enters lane l+1 at its lowest limb, which is
-      // inside the window whenever the carry is nonzero; lane 31's is dropped
-      uint32_t cin = __shfl_up_sync(~0u, c, 1);
-      if (lane == 0) cin = 0;
-      {
-        const unsigned long long v = (unsigned long long)x[0] + cin;
-        x[0] = (uint32_t)v;
-        uint32_t t = (uint32_t)(v >> 32);
-        // rare: the lowest limb overflowed; ripple through the lane and on
-        // into the next lanes (bounded: at most 32 rounds)
-        for (int round = 0; round < 32 && __any_sync(~0u, t != 0); round++) {
-#pragma unroll
-          for (int q = 1; q < RS; q++) {
-            const unsigned long long w = (unsigned long long)x[q] + t;
-            x[q] = (uint32_t)w;
-            t = (uint32_t)(w >> 32);
-          }
-          uint32_t up = __shfl_up_sync(~0u, t, 1);
-          if (lane == 0) up = 0;
-          const unsigned long long w = (unsigned long long)x[0] + up;
-          x[0] = (uint32_t)w;
-          t = (uint32_t)(w >> 32);
-        }
+      if (lane != 31) {  // limb n's high word is dropped
+        h += (uint32_t)(x[RS - 1] >> 32);
+        x[RS - 1] &= 0xffffffffull;
       }
-      // the digit: limb n, the last register of lane 31
-      if (lane == 31) lf.s[lf.k - i] = x[RS - 1];
+      const uint32_t up = __shfl_up_sync(~0u, h, 1);
+      if (lane != 0) x[0] += up;
+      if (__any_sync(~0u, lane == 31 && (uint32_t)x[RS - 2] == 0xffffffffu)) radix_resolve(x, lane);
+      // the digit: limb n with the carry out of the limb below, which then
+      // holds 32 bits
+      if (lane == 31) {
+        lf.s[lf.k - i] = (uint32_t)(x[RS - 1] + (x[RS - 2] >> 32));
+        x[RS - 2] &= 0xffffffffull;
+        x[RS - 1] = 0;  // the window's top limb enters the next round as zero
+      }
     }
   }
 }
@@ -145,8 +189,10 @@ __global__ void k_merge_fix(MergeDesc *d, int n, unsigned *flag) {
   flag[i] = (m.sh[0] == 0 && m.sl[m.kl - 1] == DEC_BASE - 1) ? 1u : 0u;
 }
 
-// The copies, MERGE_UNIT digits per unit, units of all nodes in one grid.
-constexpr int MERGE_UNIT = 4096;
+// The copies, MERGE_UNIT digits per unit, units of all nodes in one grid.  A
+// depth of 400,000 digits in units of 4096 kept 98 CTAs with 16 rounds each
+// busy for 12 us; in units of 1024 it spreads over the SMs.
+constexpr int MERGE_UNIT = 1024;
 __global__ void k_merge_copy(const MergeDesc *d, int n, unsigned long long units, const unsigned *flag) {
   for (unsigned long long u = blockIdx.x; u < units; u += gridDim.x) {
     int lo = 0, hi = n - 1;
