@@ -29,6 +29,7 @@ struct AddSubParams {
   uint32_t *r;               // n limbs
   unsigned long long n;
   int sub;                   // 1: a - b (|a| >= |b| over the window), 0: a + b
+  uint32_t word;             // not 0: a * word instead (limb i: low word of a_i * word plus high word of a_(i-1) * word)
   unsigned long long tiles;  // ceil(n / ADD_TILE)
   unsigned int *counter;     // zeroed before launch
   uint32_t *status;          // one word per tile, zeroed before launch
@@ -53,7 +54,13 @@ __global__ void __launch_bounds__(ADD_NT) k_addsub_win(AddSubParams p) {
 #pragma unroll
     for (int q = 0; q < ADD_PT; q++) {
       const long long i = i0 + q;
-      const uint32_t av = win_at(p.a, i), bv = win_at(p.b, i);
+      uint32_t av = win_at(p.a, i), bv;
+      if (p.word) {
+        av *= p.word;
+        bv = __umulhi(win_at(p.a, i - 1), p.word);
+      } else {
+        bv = win_at(p.b, i);
+      }
       if (p.sub) {
         const unsigned long long v = (unsigned long long)av - bv - c;
         s[q] = (uint32_t)v;
@@ -139,13 +146,16 @@ __global__ void k_top_nonzero(const uint32_t *x, unsigned long long n, unsigned 
   if ((threadIdx.x & 31) == 0 && best) atomicMax(top, best);
 }
 
-// *hi = 1 + the highest i < n where the windowed operands differ (0 if
-// they are equal over the window); *hi zeroed before launch.
+// *hi = 2 (i + 1) + (a_i > b_i) for the highest i < n where the windowed
+// operands differ (0 if they are equal over the window); *hi zeroed before
+// launch.
 __global__ void k_first_diff(WinOp a, WinOp b, unsigned long long n, unsigned long long *hi) {
   unsigned long long best = 0;
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
-       i += (unsigned long long)gridDim.x * blockDim.x)
-    if (win_at(a, (long long)i) != win_at(b, (long long)i)) best = i + 1;
+       i += (unsigned long long)gridDim.x * blockDim.x) {
+    const uint32_t x = win_at(a, (long long)i), y = win_at(b, (long long)i);
+    if (x != y) best = 2 * (i + 1) + (x > y ? 1 : 0);
+  }
   for (int o = 16; o; o >>= 1) {
     const unsigned long long t = __shfl_xor_sync(~0u, best, o);
     best = t > best ? t : best;

@@ -1882,32 +1882,41 @@ int radix_tree_core(const uint32_t *dy, size_t ylen, const bc_radix_node *nodes,
   if ((r = radix_leaves_device(lv, alpha))) return r;
   const double t_leaves = sync_secs(t_step);
   t_step = now();
-  // bottom-up merges, one depth at a time
+  // bottom-up merges, one depth after the other: the descriptors of all depths
+  // go up in one copy, the launches follow one another without a wait
+  std::vector<MergeDesc> mg;
+  struct Depth { size_t first, n; unsigned long long units; };
+  std::vector<Depth> depths;
+  std::vector<std::vector<size_t>> at_depth(maxd);
+  for (size_t i = 0; i < nn; i++)
+    if (nodes[i].child_h >= 0) at_depth[depth[i]].push_back(i);
+  for (int d = maxd - 1; d >= 0; d--) {
+    Depth dp{mg.size(), 0, 0};
+    for (size_t i : at_depth[d]) {
+      const bc_radix_node &x = nodes[i];
+      const size_t h = (size_t)x.child_h, l = (size_t)x.child_l;
+      const unsigned long long kh = nodes[h].k, kl = nodes[l].k;
+      if (kl != x.kl || kh + kl - 1 != x.k || kh == 0 || kl == 0) return fail(BC_ERR_INVALID);
+      mg.push_back({dsd + s_off[h], dsd + s_off[l], dsd + s_off[i], kh, kl, dp.units});
+      dp.units += (kh - 1 + kl + MERGE_UNIT - 1) / MERGE_UNIT;
+    }
+    dp.n = mg.size() - dp.first;
+    if (dp.n) depths.push_back(dp);
+  }
   const size_t o_flag = align256(nn * sizeof(MergeDesc));
   if ((r = dmeta.alloc(o_flag + nn * 4))) return r;
   MergeDesc *dm = (MergeDesc *)dmeta.p;
   unsigned *dflag = (unsigned *)((char *)dmeta.p + o_flag);
-  for (int d = maxd - 1; d >= 0; d--) {
-    std::vector<MergeDesc> mg;
-    unsigned long long units = 0;
-    for (size_t i = 0; i < nn; i++) {
-      const bc_radix_node &x = nodes[i];
-      if (depth[i] != d || x.child_h < 0) continue;
-      const size_t h = (size_t)x.child_h, l = (size_t)x.child_l;
-      const unsigned long long kh = nodes[h].k, kl = nodes[l].k;
-      if (kl != x.kl || kh + kl - 1 != x.k || kh == 0 || kl == 0) return fail(BC_ERR_INVALID);
-      mg.push_back({dsd + s_off[h], dsd + s_off[l], dsd + s_off[i], kh, kl, units});
-      units += (kh - 1 + kl + MERGE_UNIT - 1) / MERGE_UNIT;
-    }
-    if (mg.empty()) continue;
+  if (!mg.empty())
     CK(cudaMemcpyAsync(dm, mg.data(), mg.size() * sizeof(MergeDesc), cudaMemcpyHostToDevice, g.stream));
-    k_merge_fix<<<(unsigned)((mg.size() + 127) / 128), 128, 0, g.stream>>>(dm, (int)mg.size(), dflag);
+  for (const Depth &dp : depths) {
+    k_merge_fix<<<(unsigned)((dp.n + 127) / 128), 128, 0, g.stream>>>(dm + dp.first, (int)dp.n, dflag + dp.first);
     CK(cudaGetLastError());
-    const unsigned grid = (unsigned)std::min<unsigned long long>(units, (unsigned long long)g.sm_count * 8);
-    k_merge_copy<<<grid, 256, 0, g.stream>>>(dm, (int)mg.size(), units, dflag);
+    const unsigned grid = (unsigned)std::min<unsigned long long>(dp.units, (unsigned long long)g.sm_count * 8);
+    k_merge_copy<<<grid, 256, 0, g.stream>>>(dm + dp.first, (int)dp.n, dp.units, dflag + dp.first);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(g.stream));  // mg is rewritten for the next depth
   }
+  // every path below waits for the stream before mg goes out of scope
   if (stats)
     fprintf(stderr, "      conversion tree: products %.3f s, %zu leaves %.3f s, merges %.3f s\n", t_mul_total, lv.size(),
             t_leaves, sync_secs(t_step));
@@ -1980,30 +1989,57 @@ int trimmed_len(const uint32_t *dC, size_t CL, size_t *len) {
   return BC_OK;
 }
 
+// C = X * word, XL + 1 limbs, in device memory: one pass over X on the library
+// stream (k_addsub_win), where a product of XL by 1 limbs would take a whole
+// transform.  `scratch` (word_scratch bytes) must live until the stream has
+// been waited for; a lookback that gave up sets bit 0 of *flags.
+size_t word_scratch(size_t XL) { return 256 + align256(((XL + 1 + ADD_TILE - 1) / ADD_TILE) * 4); }
+int mul_word_device(uint32_t *C, const uint32_t *X, size_t XL, uint32_t word, char *scratch, unsigned *flags) {
+  const unsigned long long n = XL + 1, tiles = (n + ADD_TILE - 1) / ADD_TILE;
+  CK(cudaMemsetAsync(scratch, 0, word_scratch(XL), g.stream));
+  AddSubParams ap;
+  ap.a = WinOp{X, 0, (long long)XL};
+  ap.b = WinOp{X, 0, 0};
+  ap.r = C;
+  ap.n = n;
+  ap.sub = 0;
+  ap.word = word;
+  ap.tiles = tiles;
+  ap.counter = (unsigned int *)scratch;
+  ap.cout = (unsigned int *)(scratch + 4);
+  ap.flags = flags;
+  ap.status = (uint32_t *)(scratch + 256);
+  const unsigned grid = (unsigned)std::min<unsigned long long>(tiles, (unsigned long long)g.sm_count * 8);
+  k_addsub_win<<<grid, ADD_NT, 0, g.stream>>>(ap);
+  CK(cudaGetLastError());
+  return BC_OK;
+}
+
 // The power table of the conversion built in device memory: entry 0 comes
 // from the host; entry i from entry steps[i].src < i by the step the
 // reference's table construction takes (bigfloat/radix.c:156-205): times
 // 10^9 (len + 1 limbs, untrimmed), a squaring (trimmed product), or a
-// squaring then times 10^9 (trimmed square plus one limb).  The products
-// are the library's own exact products on device operands.
+// squaring then times 10^9 (trimmed square plus one limb).  The squares are
+// the library's own exact products on device operands.
 int radix_tree_pow_locked(const uint32_t *y, size_t ylen, const bc_radix_node *nodes, size_t nn, const uint32_t *t0,
                           size_t t0len, const bc_radix_pow_step *steps, int ntable, double alpha, uint32_t *out) {
   if (!g.init) return fail(BC_ERR_NOT_INIT);
   if (!y || !ylen || !nodes || !nn || !out || ntable < 1 || !t0 || !t0len || !steps) return fail(BC_ERR_INVALID);
   for (int i = 1; i < ntable; i++)
     if (steps[i].src < 0 || steps[i].src >= i || steps[i].op < 1 || steps[i].op > 3) return fail(BC_ERR_INVALID);
-  std::vector<DevBuf> tab(ntable + 1);  // the last one holds y and 10^9
+  std::vector<DevBuf> tab(ntable + 1);  // the last one holds y
+  std::vector<DevBuf> wscratch(ntable);  // of the products by 10^9
+  DevBuf wflag;
   std::vector<size_t> tlen(ntable);
   std::vector<const uint32_t *> dtab(ntable);
   int r;
   const size_t ypad = (ylen + 63) & ~size_t(63);
-  if ((r = tab[ntable].alloc((ypad + 64) * 4))) return r;
-  uint32_t *dy = (uint32_t *)tab[ntable].p, *dbase = dy + ypad;
+  if ((r = tab[ntable].alloc(ypad * 4)) || (r = wflag.alloc(4))) return r;
+  CK(cudaMemsetAsync(wflag.p, 0, 4, g.stream));
+  uint32_t *dy = (uint32_t *)tab[ntable].p;
   {
     std::vector<SpanJob> jobs{{0, (char *)y, ylen * 4}};
     if ((r = stage_h2d((char *)dy, jobs, ylen * 4))) return r;
-    const uint32_t nine = DEC_BASE;
-    CK(cudaMemcpyAsync(dbase, &nine, 4, cudaMemcpyHostToDevice, g.stream));
   }
   if ((r = tab[0].alloc(t0len * 4))) return r;
   CK(cudaMemcpyAsync(tab[0].p, t0, t0len * 4, cudaMemcpyHostToDevice, g.stream));
@@ -2018,9 +2054,8 @@ int radix_tree_pow_locked(const uint32_t *y, size_t ylen, const bc_radix_node *n
     const size_t XL = tlen[j];
     if (op == 1) {  // times 10^9
       const size_t CL = XL + 1;
-      if ((r = tab[i].alloc(CL * 4))) return r;
-      bc_mul_desc d{(uint32_t *)tab[i].p, CL, X, XL, dbase, 1};
-      if ((r = mul_batch_locked(&d, 1, &st, nullptr, BC_BATCH_DEVICE_OPERANDS))) return r;
+      if ((r = tab[i].alloc(CL * 4)) || (r = wscratch[i].alloc(word_scratch(XL)))) return r;
+      if ((r = mul_word_device((uint32_t *)tab[i].p, X, XL, DEC_BASE, (char *)wscratch[i].p, (unsigned *)wflag.p))) return r;
       tlen[i] = CL;
     } else {
       const size_t CL = 2 * XL;
@@ -2035,14 +2070,18 @@ int radix_tree_pow_locked(const uint32_t *y, size_t ylen, const bc_radix_node *n
         sq.p = nullptr;
         tlen[i] = L;
       } else {  // then times 10^9 into L + 1 limbs
-        if ((r = tab[i].alloc((L + 1) * 4))) return r;
-        bc_mul_desc d2{(uint32_t *)tab[i].p, L + 1, (const uint32_t *)sq.p, L, dbase, 1};
-        if ((r = mul_batch_locked(&d2, 1, &st, nullptr, BC_BATCH_DEVICE_OPERANDS))) return r;
+        if ((r = tab[i].alloc((L + 1) * 4)) || (r = wscratch[i].alloc(word_scratch(L)))) return r;
+        if ((r = mul_word_device((uint32_t *)tab[i].p, (const uint32_t *)sq.p, L, DEC_BASE, (char *)wscratch[i].p, (unsigned *)wflag.p)))
+          return r;
         tlen[i] = L + 1;
       }
     }
     dtab[i] = (const uint32_t *)tab[i].p;
   }
+  unsigned gave_up = 0;
+  CK(cudaMemcpyAsync(&gave_up, wflag.p, 4, cudaMemcpyDeviceToHost, g.stream));
+  CK(cudaStreamSynchronize(g.stream));
+  if (gave_up) return fail(BC_ERR_TIMEOUT);
   if (getenv("BC_STATS")) {
     cudaStreamSynchronize(g.stream);
     fprintf(stderr, "      conversion power table: %d entries, %.3f s\n", ntable,
@@ -2156,6 +2195,7 @@ int dnum_uaddsub(DNum &t, const DNum &a, const DNum &b, size_t p, bool sub) {
   ap.r = (uint32_t *)c.p;
   ap.n = (unsigned long long)n;
   ap.sub = sub ? 1 : 0;
+  ap.word = 0;
   ap.tiles = tiles;
   ap.counter = (unsigned int *)sp;
   ap.cout = (unsigned int *)(sp + 4);
@@ -2222,15 +2262,7 @@ int dnum_ucmp(const DNum &a, const DNum &b, int *res) {
   unsigned long long hi = 0;
   CK(cudaMemcpyAsync(&hi, dhi, 8, cudaMemcpyDeviceToHost, g.stream));
   CK(cudaStreamSynchronize(g.stream));
-  if (!hi) {
-    *res = 0;
-    return BC_OK;
-  }
-  const long long i = (long long)hi - 1;
-  uint32_t x = 0, y = 0;
-  if (i >= wa.lo && i < wa.hi) CK(cudaMemcpy(&x, wa.x + (i - wa.lo), 4, cudaMemcpyDeviceToHost));
-  if (i >= wb.lo && i < wb.hi) CK(cudaMemcpy(&y, wb.x + (i - wb.lo), 4, cudaMemcpyDeviceToHost));
-  *res = x > y ? 1 : -1;
+  *res = hi == 0 ? 0 : ((hi & 1) ? 1 : -1);
   return BC_OK;
 }
 
@@ -2328,6 +2360,7 @@ int selftest_wait_locked(double *secs) {
   ap.r = (uint32_t *)(bp + o_r);
   ap.n = n;
   ap.sub = 0;
+  ap.word = 0;
   ap.tiles = 2;
   ap.counter = (unsigned int *)(bp + o_sc);
   ap.cout = (unsigned int *)(bp + o_sc + 4);
