@@ -109,26 +109,31 @@ template <int L> struct Pass16 {
   static constexpr int MINB = 384 / NT;
   // dynamic shared memory
   static constexpr size_t TWB = (size_t)L * 16;  // block16 twiddles
-  static constexpr size_t SMEM_INV = 2 * (size_t)L * W * 16 + TWB + (size_t)L * 16 + 2 * 36 * 16 + 1024;
+  static constexpr size_t SMEM_INV = 2 * (size_t)L * W * 16 + TWB + (size_t)L * 16 + 2 * 38 * 16 + 1024;
   static constexpr size_t SMEM_FWD = (size_t)L * W * 16 + (size_t)PackTile<L>::STAGE_WORDS * 4 + TWB +
-                                     (size_t)L * 16 + 2 * 36 * 16 + 1024;
+                                     (size_t)L * 16 + 2 * 38 * 16 + 1024;
 };
 
 // Outer-pass twiddles e^{-2 pi i col (4 k1 - 1)/(4M)} of one thread, for
-// k1 = t + R i (i = 0..15) and col = tile W + s, as two runs of 8 (a base
+// k1 = t + R i (i = 0..15) and col = tile W + s, as four runs of 4 (a base
 // and a step, then products).  With T(m) = e^{-2 pi i m/(4M)} (m signed) and
 // T(col x) = T(tile W x) T(s x):
-//   base of the first run   T(col (4t - 1))     = F_t       * T(s (4t - 1))
-//   step                    T(col 4R)           = G         * T(s 4R)
-//   base of the second run  T(col (4t + 32R - 1)) = base1 * H * T(s 32R)
-// The tile factors F_t (t < 16), G = T(tile W 4R), H = T(tile W 32R) come
-// from the two-level table, T(m) = lo * hi: 18 threads copy both entries of
-// theirs to shared memory one unit ahead (cp.async), each thread multiplies
-// the three it needs.  The column factors depend only on the thread (s, t
-// fixed by tid) and stay in registers.  Computing the tile factors by
-// sincospi took 130 instructions in every warp of every unit, a tenth of the
-// pass's issue slots, and at the start of a CTA 2 us.
-constexpr int TILE_TW = 18;            // tile factors per unit
+//   base of run 0      T(col (4t - 1))          = F_t * T(s (4t - 1))
+//   step               T(col 4R)                = G * T(s 4R)
+//   base of run j      that of run j - 1 or 0 times T(col 16R j), j = 1, 2
+//   T(col 16R) = J * T(s 16R), T(col 32R) = H * T(s 32R)
+// The tile factors F_t (t < 16), G, J, H come from the two-level table, T(m) =
+// lo * hi: both entries of each are copied to shared memory one unit ahead
+// (cp.async), each thread multiplies the four pairs it needs.  The column
+// factors depend only on the thread (s, t fixed by tid) and stay in registers.
+// Computing the tile factors by sincospi took 130 instructions in every warp
+// of every unit, a tenth of the pass's issue slots, and at the start of a CTA
+// 2 us.  The runs are short because a table product's error is above
+// sincospi's and grows along a run: with two runs of 8 the rounding error of a
+// 2^24-limb product grew from 0.0142 to 0.0158, with four of 4 it is @E.
+// (Steps per column straight from the table, one product each, 0.0135, took
+// 64 entries a unit and the inverse pass from 0.233 to 0.247 ms.)
+constexpr int TILE_TW = 19;             // tile factors per unit
 constexpr int TILE_TW_N = 2 * TILE_TW;  // their table entries (lo, hi)
 
 // Index of T(m) = e^{-2 pi i m/(4M)} in the two-level table, |m| < 4M.
@@ -137,37 +142,46 @@ __device__ __forceinline__ unsigned long long t4m_index(long long m, int M) {
 }
 
 struct ColTw16 {
-  double2 c0, cst, cb1;
+  double2 c0, cst, cj, ch;
 };
 template <int R>
 __device__ __forceinline__ ColTw16 col_tw16(int s, int t, const Tw2 &T, int M) {
   ColTw16 c;
   c.c0 = tw2_get(T, t4m_index((long long)s * (4 * t - 1), M));
   c.cst = tw2_get(T, (unsigned long long)s * 4 * R);
-  c.cb1 = tw2_get(T, (unsigned long long)s * 32 * R);
+  c.cj = tw2_get(T, (unsigned long long)s * 16 * R);
+  c.ch = tw2_get(T, (unsigned long long)s * 32 * R);
   return c;
 }
 
-// Copies the table entries of tile's factors to fac[0..35] (lo and hi of
-// factor j at 2j and 2j + 1); the caller commits, waits and synchronises.
+// Copies the table entries of tile's factors to fac (lo of factor j at j, hi
+// at TILE_TW + j: F_0..F_15, G, J, H); the caller commits, waits and
+// synchronises.
 template <int R, int W>
 __device__ __forceinline__ void tile_tw16(double2 *fac, int tile, const Tw2 &T, int M) {
-  const int j = threadIdx.x >> 1;
-  if (j < TILE_TW) {
-    const long long x = j < 16 ? 4 * j - 1 : (j == 16 ? 4 * R : 32 * R);
+  const int k = threadIdx.x;
+  if (k < TILE_TW_N) {
+    const int j = k < TILE_TW ? k : k - TILE_TW;
+    const long long x = j < 16 ? 4 * j - 1 : (j == 16 ? 4 * R : (j == 17 ? 16 * R : 32 * R));
     const unsigned long long m = t4m_index((long long)tile * W * x, M);
-    cp_async16(fac + threadIdx.x, (threadIdx.x & 1) ? &T.hi[m >> T.h] : &T.lo[m & T.mask], 16);
+    cp_async16(fac + k, k < TILE_TW ? &T.lo[m & T.mask] : &T.hi[m >> T.h], 16);
   }
 }
 
+// The bases of the four runs and the step.
 struct OuterRun16 {
-  double2 b0, b1, st;
+  double2 b[4], st;
 };
+template <int R>
 __device__ __forceinline__ OuterRun16 outer_run16(const double2 *fac, const ColTw16 &c, int t) {
+  auto factor = [&](int j) { return cmul(fac[j], fac[TILE_TW + j]); };
   OuterRun16 o;
-  o.b0 = cmul(cmul(fac[2 * t], fac[2 * t + 1]), c.c0);
-  o.st = cmul(cmul(fac[32], fac[33]), c.cst);
-  o.b1 = cmul(o.b0, cmul(cmul(fac[34], fac[35]), c.cb1));
+  const double2 j = cmul(factor(17), c.cj);
+  o.b[0] = cmul(factor(t), c.c0);
+  o.b[1] = cmul(o.b[0], j);
+  o.b[2] = cmul(o.b[0], cmul(factor(18), c.ch));
+  o.b[3] = cmul(o.b[2], j);
+  o.st = cmul(factor(16), c.cst);
   return o;
 }
 
@@ -286,11 +300,11 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(c
     if (un < total) stage_copy(un, par ^ 1);
     cp_async_commit();
     block16<L, W, false>(v, t, s, tile, twS);
-    const OuterRun16 tw = outer_run16(fac + par * TILE_TW_N, ct, t);
-    double2 w = tw.b0;
+    const OuterRun16 tw = outer_run16<R>(fac + par * TILE_TW_N, ct, t);
+    double2 w = tw.b[0];
 #pragma unroll
     for (int i = 0; i < P16; i++) {
-      if (i == 8) w = tw.b1;
+      if (i % 4 == 0) w = tw.b[i / 4];
       gbuf[(unsigned)(t + i * R) * (unsigned)p.S1 + col] = cmul(v[i], w);
       w = cmul(w, tw.st);
     }
@@ -361,11 +375,11 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB)
     double2 *bf = buf0 + st * L * W;
     double2 v[P16];
     {
-      const OuterRun16 tw = outer_run16(fac + st * TILE_TW_N, ct, t);
-      double2 w = tw.b0;
+      const OuterRun16 tw = outer_run16<R>(fac + st * TILE_TW_N, ct, t);
+      double2 w = tw.b[0];
 #pragma unroll
       for (int i = 0; i < P16; i++) {
-        if (i == 8) w = tw.b1;
+        if (i % 4 == 0) w = tw.b[i / 4];
         v[i] = cmulc(bf[bidx<L>(t + i * R, s)], w);
         w = cmul(w, tw.st);
       }

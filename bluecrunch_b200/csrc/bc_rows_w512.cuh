@@ -11,13 +11,12 @@
 // The transform, with n = l + 32 i (l = lane) and k = k1 + 16 k2:
 //   1. DFT-16 over i in registers: Y[l][k1];
 //   2. twiddle e^{-2 pi i l k1/512};
-//   3. the remaining DFT-32 over l, split l = l1 + 16 l0 and
-//      k2 = 2 k2' + e: lanes l1 and l1 + 16 swap their 16 values by shuffle
-//      and form B_e = A_l1 + (-1)^e A_(l1+16) (e = the lane's half), then the
-//      upper half multiplies by e^{-2 pi i l1/32};
-//   4. one transpose inside each half-warp through shared memory, so that
-//      lane L = k1 + 16 e holds B_e(l1, k1) for l1 = 0..15;
-//   5. DFT-16 over l1 in registers: v[k2'] = X[k1 + 16 (2 k2' + e)] =
+//   3. one transpose through shared memory: lane L = k1 + 16 e reads all 32
+//      values A_l of its k1 (the two lanes of a k1 the same ones) and does the
+//      first radix-2 step of the remaining DFT-32 over l as they arrive:
+//      B_e(l1) = A_l1 + (-1)^e A_(l1+16), l1 = 0..15, k2 = 2 k2' + e; the
+//      lanes with e = 1 multiply by e^{-2 pi i l1/32} (constants);
+//   4. DFT-16 over l1 in registers: v[k2'] = X[k1 + 16 (2 k2' + e)] =
 //      X[L + 32 k2'].
 // The spectrum lands in the layout the points came in, so A and B meet lane
 // by lane, and the same steps on conjugate roots give the inverse.
@@ -43,21 +42,22 @@ __device__ __forceinline__ void row_dft512(double2 (&v)[R5_P], int lane, double2
   dft16<INV>(v);  // over i: v[k1] = Y[lane][k1]
 #pragma unroll
   for (int k1 = 1; k1 < R5_P; k1++) v[k1] = ctw<INV>(v[k1], twT[k1 * 32 + lane]);
-  const bool upper = lane >= 16;
-  const double2 w = twT[(lane & 15) * 32 + 16];  // e^{-2 pi i 16 l1/512} = e^{-2 pi i l1/32}
-#pragma unroll
-  for (int k1 = 0; k1 < R5_P; k1++) {
-    const double2 o = make_double2(__shfl_xor_sync(0xffffffffu, v[k1].x, 16), __shfl_xor_sync(0xffffffffu, v[k1].y, 16));
-    const double2 b = upper ? make_double2(o.x - v[k1].x, o.y - v[k1].y) : make_double2(v[k1].x + o.x, v[k1].y + o.y);
-    v[k1] = upper ? ctw<INV>(b, w) : b;
-  }
 #pragma unroll
   for (int k1 = 0; k1 < R5_P; k1++) buf[lane * 16 + (k1 ^ (lane & 15))] = v[k1];
   __syncwarp();
-  const int k1 = lane & 15, h = lane & 16;
+  const int k1 = lane & 15;
+  const bool odd = lane >= 16;
+  const double sg = odd ? -1.0 : 1.0;
 #pragma unroll
-  for (int l1 = 0; l1 < R5_P; l1++) v[l1] = buf[(l1 + h) * 16 + (k1 ^ l1)];
+  for (int l1 = 0; l1 < R5_P; l1++) {
+    const double2 a = buf[l1 * 16 + (k1 ^ l1)], b = buf[(l1 + 16) * 16 + (k1 ^ l1)];
+    v[l1] = make_double2(fma(sg, b.x, a.x), fma(sg, b.y, a.y));
+  }
   __syncwarp();  // the buffer is free for the next transform
+  if (odd) {
+#pragma unroll
+    for (int l1 = 1; l1 < R5_P; l1++) v[l1] = rot32<INV>(v[l1], l1);
+  }
   dft16<INV>(v);  // over l1: v[k2'] = X[lane + 32 k2']
 }
 
