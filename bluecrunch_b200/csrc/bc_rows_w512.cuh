@@ -61,17 +61,21 @@ __device__ __forceinline__ void row_dft512(double2 (&v)[R5_P], int lane, double2
   dft16<INV>(v);  // over l1: v[k2'] = X[lane + 32 k2']
 }
 
-// Occupancy: the kernel holds about 250 registers per thread (a row's 16
-// points, the DFT-16 temporaries and the twiddles it loads ahead), so two
-// CTAs of four warps share an SM; three CTAs (170 registers) spill and
-// measured slower.
+// What bounds it: shared memory (0.75 of the LSU data path's rate: per row and
+// transform one read of the row, the twiddles, the transpose's write and twice
+// its read).  So B's spectrum stays in registers while A is transformed (255
+// of them, no spills; parked in shared memory it cost 128 of 1,166 passes per
+// row: 0.343 -> 0.334 ms at 2^25 points).  Two CTAs of four warps share an SM;
+// three (168 registers) or two of five measured the same or slower.  Loading 6
+// of the 15 twiddles and multiplying the others took 0.331 ms, but raised the
+// rounding error of 2^18-point products by a tenth.
 // Grid: persistent, R5_WARPS warps per CTA; warp w of CTA c takes rows
 // c*R5_WARPS + w + k*gridDim.x*R5_WARPS of the class (row q of item i is
-// bufA + q*512).  Buffers, copies and waits as in k2_rows_w1024: without
-// squaring, B's spectrum is parked in buffer 1 and B's next row lands there
-// during the inverse transform, A's next row in buffer 0 likewise; squaring
-// alternates its rows between the two buffers.  The tensor maps of the
-// generic row kernel's signature are not used.
+// bufA + q*512).  Copies and waits as in k2_rows_w1024: without squaring, B's
+// next row lands in buffer 1 from the end of B's transform on, A's next row in
+// buffer 0 after the inverse transform; squaring alternates its rows between
+// the two buffers.  The tensor maps of the generic row kernel's signature are
+// not used.
 template <bool SQ>
 __global__ void __launch_bounds__(32 * R5_WARPS, 2)
     k2_rows_w512(ClassParams p, const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap) {
@@ -159,28 +163,24 @@ __global__ void __launch_bounds__(32 * R5_WARPS, 2)
     }
     for (; r < total; r += stride) {
       const bool more = r + stride < total;
-      double2 v[R5_P];
-      // B: forward transform, spectrum parked in buffer 1 (natural order)
-      if (!take(v, buf1, bar1, ph1)) {
+      double2 v[R5_P], sb[R5_P];
+      // B: forward transform, its spectrum stays in registers
+      if (!take(sb, buf1, bar1, ph1)) {
         drain = 3u;  // A's row r is in flight too
         bad_row = r;
         break;
       }
-      row_dft512<false>(v, lane, buf1, twT);
-#pragma unroll
-      for (int i = 0; i < R5_P; i++) buf1[lane + 32 * i] = v[i];
-      // A: forward transform, product with B's spectrum (each lane reads
-      // back only the entries it wrote)
+      row_dft512<false>(sb, lane, buf1, twT);
+      if (more) fetch(buf1, bar1, r + stride, true);
+      // A: forward transform, product with B's spectrum lane by lane
       if (!take(v, buf0, bar0, ph0)) {
-        drain = 1u;  // B's next row is not issued yet
+        drain = 1u | (more ? 2u : 0u);  // B's next row is in flight
         bad_row = r;
         break;
       }
       row_dft512<false>(v, lane, buf0, twT);
 #pragma unroll
-      for (int i = 0; i < R5_P; i++) v[i] = cmul(v[i], buf1[lane + 32 * i]);
-      __syncwarp();
-      if (more) fetch(buf1, bar1, r + stride, true);
+      for (int i = 0; i < R5_P; i++) v[i] = cmul(v[i], sb[i]);
       row_dft512<true>(v, lane, buf0, twT);
       if (more) fetch(buf0, bar0, r + stride, false);
       double2 *const ra = row_base(r, false);
