@@ -505,9 +505,10 @@ KInfo small_info() {
 }
 
 template <int L>
-KInfo outer_fwd16_info() {
+KInfo outer_fwd16_info(int parts) {
   using T = Pass16<L>;
-  KInfo k{(const void *)k3_outer_fwd<L>, T::NT, T::SMEM_FWD, "outer_fwd", SIG_P};
+  KInfo k{parts == 1 ? (const void *)k3_outer_fwd<L, 1> : (const void *)k3_outer_fwd<L, 2>, T::NT, T::SMEM_FWD(parts),
+          "outer_fwd", SIG_P};
   k.pts = P16;
   return k;
 }
@@ -520,12 +521,12 @@ KInfo outer_inv16_info() {
   return k;
 }
 
-KInfo get_outer(int L, bool inv) {
+KInfo get_outer(int L, bool inv, int parts = 2) {
   if (g.pass16) {
     switch (L) {
-      case 64: return inv ? outer_inv16_info<64>() : outer_fwd16_info<64>();
-      case 128: return inv ? outer_inv16_info<128>() : outer_fwd16_info<128>();
-      case 256: return inv ? outer_inv16_info<256>() : outer_fwd16_info<256>();
+      case 64: return inv ? outer_inv16_info<64>() : outer_fwd16_info<64>(parts);
+      case 128: return inv ? outer_inv16_info<128>() : outer_fwd16_info<128>(parts);
+      case 256: return inv ? outer_inv16_info<256>() : outer_fwd16_info<256>(parts);
     }
   }
   switch (L) {
@@ -764,7 +765,7 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
     return launch(n * kc.cluster <= 2 * g.sm_count ? kc : get_small(s.M, sq), n, params, nl, stream, timed);
   }
   const cuuint64_t M16 = (cuuint64_t)s.M * 16, S1 = (cuuint64_t)params.S1, Lr = (cuuint64_t)params.Lr;
-  KInfo ko = get_outer(s.L1, false), ki = get_outer(s.L1, true);
+  KInfo ko = get_outer(s.L1, false, params.parts == 1 ? 1 : 2), ki = get_outer(s.L1, true);
   const int W1 = ko.threads / (s.L1 / ko.pts);
   ClassParams p = params;
   p.fd_outer = FastDiv((uint32_t)(S1 / W1));
@@ -1506,8 +1507,10 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     unsigned long long tiles = 0;
     bool w16 = true;  // every item of the class has width 16: the carry pass specialised for it
     for (size_t k = first; k < first + n; k++) {
-      tiles += works[order[k]]->pl.ntiles;
-      w16 = w16 && works[order[k]]->pl.b == 16;
+      const Plan &pk = works[order[k]]->pl;
+      tiles += pk.ntiles;
+      w16 = w16 && pk.b == 16;
+      if (pk.ndA > (size_t)s.M || (!sq && pk.ndB > (size_t)s.M)) p.parts = 2;
     }
     p.carry_tiles = tiles;
     const ClassSlab &cs = slab[c.first];
@@ -1523,6 +1526,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   for (int k = 0; k < nstreams; k++) {
     CK(cudaEventRecord(g.class_ev[k], g.class_stream[k]));
     CK(cudaStreamWaitEvent(lstream, g.class_ev[k], 0));
+    p.parts = 1;
   }
   if (graph) {
     cudaGraph_t gr = nullptr;
@@ -3220,3 +3224,4 @@ extern "C" int bc_gpu_mul_noalloc(uint32_t *C, size_t CL, const uint32_t *A, siz
   }
   return fail(BC_ERR_PRECISION);
 }
+    p.parts = pl.ndA > M || (!square && pl.ndB > M) ? 2 : 1;

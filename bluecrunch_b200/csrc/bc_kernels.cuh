@@ -79,6 +79,7 @@ struct ClassParams {
   const ItemDesc *items;
   int nitems;
   int sq;                 // every item of the class squares (one operand)
+  int parts;              // 2 when an operand of the class has digits at M or above (imaginary parts), else 1
   unsigned int *counter;  // k_carry dynamic tile counter (zeroed before launch)
   unsigned long long carry_tiles;  // total k_carry tiles over the class
   // fused middle pass (three levels): per block (nitems * L1 of them) the

@@ -107,11 +107,16 @@ template <int L> struct Pass16 {
   static_assert(L == 64 || L == 128 || L == 256, "16-point passes cover L1 = 64, 128, 256");
   // twelve warps per SM (at most 170 registers per thread)
   static constexpr int MINB = 384 / NT;
+  // the forward pass of operands without digits at M or above (no imaginary
+  // parts, half the limb stage): sixteen (128 registers; L = 64 would spill)
+  static constexpr int MINB_FWD(int parts) { return parts == 1 && L > 64 ? 512 / NT : MINB; }
   // dynamic shared memory
   static constexpr size_t TWB = (size_t)L * 16;  // block16 twiddles
   static constexpr size_t SMEM_INV = 2 * (size_t)L * W * 16 + TWB + (size_t)L * 16 + 2 * 38 * 16 + 1024;
-  static constexpr size_t SMEM_FWD = (size_t)L * W * 16 + (size_t)PackTile<L>::STAGE_WORDS * 4 + TWB +
-                                     (size_t)L * 16 + 2 * 38 * 16 + 1024;
+  static constexpr size_t SMEM_FWD(int parts) {
+    return (size_t)L * W * 16 + (size_t)PackTile<L>::STAGE_WORDS / 2 * parts * 4 + TWB + (size_t)L * 16 + 2 * 38 * 16 +
+           1024;
+  }
 };
 
 // Outer-pass twiddles e^{-2 pi i col (4 k1 - 1)/(4M)} of one thread, for
@@ -189,8 +194,12 @@ __device__ __forceinline__ OuterRun16 outer_run16(const double2 *fac, const ColT
 // Units: (item, operand, column tile), as k2_outer_fwd.  One limb stage: the
 // next unit's words are copied (cp.async) as soon as this unit's digits are
 // cut, and land while this unit is transformed and stored.
-template <int L>
-__global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(const __grid_constant__ ClassParams p) {
+// PARTS: 1 when no operand of the class has digits at M or above (products of
+// operands of about one length), so the limb stage holds one part and four
+// CTAs of 128 threads fit an SM instead of three: 0.360 ms against 0.380 at 2^25
+// points.
+template <int L, int PARTS>
+__global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB_FWD(PARTS)) k3_outer_fwd(const __grid_constant__ ClassParams p) {
   pdl_trigger();  // the first pass of a class: launched normally, lets the next one start early
   using T = Pass16<L>;
   using K = PackTile<L>;
@@ -198,8 +207,8 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(c
   static_assert(K::W == W, "pack tile geometry");
   extern __shared__ unsigned char smraw[];
   double2 *tile = align1024(smraw);
-  uint32_t *stg = reinterpret_cast<uint32_t *>(tile + L * W);  // one stage of STAGE_WORDS
-  double2 *twS = reinterpret_cast<double2 *>(stg + K::STAGE_WORDS);
+  uint32_t *stg = reinterpret_cast<uint32_t *>(tile + L * W);  // one stage: L segments per part
+  double2 *twS = reinterpret_cast<double2 *>(stg + K::STAGE_WORDS / 2 * PARTS);
   double2 *pwS = twS + L;
   double2 *fac = pwS + L;  // tile factors of a unit, of the units in turn at fac + par * TILE_TW_N
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
@@ -224,7 +233,7 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(c
     const bool al16 = it.al16;
     const int RW = (int)((unsigned)p.S1 * (unsigned)b / 32), PW = (int)((unsigned)p.M * (unsigned)b / 32);
     const int wbase = ((tl * W * b) >> 5) - 1 - seg_shift(tl, b, al16);
-    const int parts = it.nd > (unsigned)p.M ? 2 : 1;
+    const int parts = PARTS == 2 && it.nd > (unsigned)p.M ? 2 : 1;
     if (al16) {
       constexpr int CH = K::SEGW4 / 4;
       const int NCH = parts * L * CH;
@@ -270,7 +279,7 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB) k3_outer_fwd(c
                          (unsigned)(s * b);  // bit of digit j0+s in its staged segment
     const unsigned wi = (rel - 1) >> 5, sh = (rel - 1) & 31;
     const unsigned mask = (1u << b) - 1;
-    const bool imag = nd > (unsigned)p.M;
+    const bool imag = PARTS == 2 && nd > (unsigned)p.M;
     auto digit = [&](int part, int n1) -> double {
       const unsigned j = (unsigned)n1 * (unsigned)p.S1 + col + (part ? (unsigned)p.M : 0u);
       const uint32_t *rw = stg + (part * L + n1) * K::SEGW4 + wi;
