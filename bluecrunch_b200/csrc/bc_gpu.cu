@@ -33,6 +33,7 @@
 #include "bc_radix.cuh"
 #include "bc_rows_warp.cuh"
 #include "bc_rows_w512.cuh"
+#include "bc_rows2.cuh"
 #include "bc_arith.cuh"
 #include "bc_pass16.cuh"
 #include "bc_block.cuh"
@@ -469,7 +470,8 @@ struct KInfo {
   int box = 0;            // TMA box lines (rows) the kernel expects per box
   unsigned unit_bytes = 0; // bytes the kernel waits for per staged unit (per operand)
   int parts = 1;          // boxes per column group (or per row)
-  bool warp_rows = false; // a row kernel with one warp per row and no tensor maps
+  bool warp_rows = false; // a row kernel without tensor maps (bulk copies of whole rows)
+  int rows = 0;           // rows per unit of such a kernel (0: one per warp)
   int pts = PTS;          // points per thread of a column pass (tile width = threads / (L / pts))
   int cluster = 1;        // CTAs per cluster (units are clusters)
   bool coop = false;      // cooperative launch: every CTA resident (its warps wait on one another)
@@ -546,6 +548,16 @@ KInfo get_mid(int L, bool inv) {
   }
   return {};
 }
+template <int L, bool SQ>
+KInfo rows2_info() {
+  using T = Rows2<L>;
+  KInfo k{(const void *)k5_rows<L, SQ>, T::NT, T::SMEM, "rows", SIG_P_MAP2};
+  k.warp_rows = true;
+  k.rows = T::NR;
+  return k;
+}
+#define ROW2CASE(L) \
+  case L: return sq ? rows2_info<L, true>() : rows2_info<L, false>();
 #define ROWCASE(L) \
   case L: return sq ? rows_info<L, true>() : rows_info<L, false>();
 KInfo get_rows(int L, bool sq) {
@@ -560,6 +572,11 @@ KInfo get_rows(int L, bool sq) {
             "rows", SIG_P_MAP2};
     k.warp_rows = true;
     return k;
+  }
+  if (g.rows_warp) {
+    switch (L) {
+      ROW2CASE(128) ROW2CASE(192) ROW2CASE(256) ROW2CASE(320) ROW2CASE(384)
+    }
   }
   switch (L) {
     ROWCASE(128) ROWCASE(192) ROWCASE(256) ROWCASE(320) ROWCASE(384) ROWCASE(512) ROWCASE(640) ROWCASE(768)
@@ -716,7 +733,8 @@ bool shape_launch_ok(const Shape &s, bool sq) {
   if (S1 % W1 || W1 % 8 || ki.threads / (s.L1 / ki.pts) != W1) return false;
   if ((size_t)(W1 / 8) * ki.parts * 128 * ki.box != ki.unit_bytes || (size_t)ki.box * ki.parts != (size_t)s.L1)
     return false;
-  const int NR = kr.warp_rows ? 1 : kr.threads / ((int)Lr / PTS);
+  const int NR = kr.rows ? kr.rows : (kr.warp_rows ? 1 : kr.threads / ((int)Lr / PTS));
+  if (kr.rows && (s.M / Lr) % NR != 0) return false;
   if (!kr.warp_rows && ((size_t)kr.parts * 128 * kr.box * NR != kr.unit_bytes || (size_t)kr.box * kr.parts != Lr / 8 ||
                         (s.M / Lr) % NR != 0 || kr.box > 256 || kr.box % 8))
     return false;
@@ -826,7 +844,7 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
       // one warp per row, plain loads and stores: no tensor maps
       KInfo kr = get_rows(s.Lr, sq);
       const long long rows = n * (long long)(s.M / s.Lr);
-      const long long wpc = kr.threads / 32;  // rows (warps) per CTA
+      const long long wpc = kr.rows ? kr.rows : kr.threads / 32;  // rows per CTA and unit
       if ((r = launch(kr, (rows + wpc - 1) / wpc, p, nl, stream, timed, nullptr, nullptr, pdl))) return r;
     } else {
       KInfo kr = get_rows(s.Lr, sq);
@@ -1506,6 +1524,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     }
     unsigned long long tiles = 0;
     bool w16 = true;  // every item of the class has width 16: the carry pass specialised for it
+    p.parts = 1;
     for (size_t k = first; k < first + n; k++) {
       const Plan &pk = works[order[k]]->pl;
       tiles += pk.ntiles;
@@ -1526,7 +1545,6 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   for (int k = 0; k < nstreams; k++) {
     CK(cudaEventRecord(g.class_ev[k], g.class_stream[k]));
     CK(cudaStreamWaitEvent(lstream, g.class_ev[k], 0));
-    p.parts = 1;
   }
   if (graph) {
     cudaGraph_t gr = nullptr;
@@ -3207,6 +3225,7 @@ extern "C" int bc_gpu_mul_noalloc(uint32_t *C, size_t CL, const uint32_t *A, siz
     p.sq = square ? 1 : 0;
     p.counter = ctr;
     p.carry_tiles = pl.ntiles;
+    p.parts = pl.ndA > M || (!square && pl.ndB > M) ? 2 : 1;
     p.nb = square ? 0 : 1;  // one B slot, its own (bowner null)
     size_t nl = 0;
     int r = launch_class(s, square, p, 1, pl.ntiles, it.bufA, it.bufB, stream, false, &nl);
@@ -3224,4 +3243,3 @@ extern "C" int bc_gpu_mul_noalloc(uint32_t *C, size_t CL, const uint32_t *A, siz
   }
   return fail(BC_ERR_PRECISION);
 }
-    p.parts = pl.ndA > M || (!square && pl.ndB > M) ? 2 : 1;
