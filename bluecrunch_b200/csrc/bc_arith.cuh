@@ -7,7 +7,8 @@
 // _bigfloat_word_at over the window [bot, top) (bigfloat/addsub.c:17-27,
 // 65-181).  The carry (borrow) chain is resolved like the carry of k_add:
 // each thread's limbs map a carry in of 0 or 1 to a carry out, a CTA scans the
-// maps, and tiles chain by decoupled lookback with bounded waits.
+// maps, and tiles chain by decoupled lookback with bounded waits (a status
+// word carries all that it says, so it needs no ordering of other memory).
 #pragma once
 #include <cuda/atomic>
 
@@ -80,17 +81,17 @@ __global__ void __launch_bounds__(ADD_NT) k_addsub_win(AddSubParams p) {
       cuda::atomic_ref<uint32_t, cuda::thread_scope_device> me(p.status[tile]);
       int cin = 0;
       if (tile == 0) {
-        me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_release);
+        me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_relaxed);
       } else {
-        if (fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_release);
-        else me.store(ST_AGG | agg, cuda::memory_order_release);
+        if (fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_relaxed);
+        else me.store(ST_AGG | agg, cuda::memory_order_relaxed);
         uint32_t acc = FN_ID;
         long long prev = (long long)tile - 1;
         int spins = 0;
         bool timed_out = false;
         for (;;) {
           cuda::atomic_ref<uint32_t, cuda::thread_scope_device> st(p.status[prev]);
-          const uint32_t v = st.load(cuda::memory_order_acquire);
+          const uint32_t v = st.load(cuda::memory_order_relaxed);
           if (v & ST_INC) {
             cin = fn_apply(acc, (int)(v & 3u) - 1);
             break;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(ADD_NT) k_addsub_win(AddSubParams p) {
           atomicOr(p.flags, 1u);
           cin = 0;
         }
-        if (!fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, cin) + 1), cuda::memory_order_release);
+        if (!fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, cin) + 1), cuda::memory_order_relaxed);
       }
       s_cin = cin;
     }

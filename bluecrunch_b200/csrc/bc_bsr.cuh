@@ -75,34 +75,33 @@ __global__ void __launch_bounds__(32 * WLEAF_WARPS) k_bsr_leaves_wide(uint32_t a
   if (__any_sync(~0u, ovf != 0) && lane == 0) atomicOr(flags, 1u);
 }
 
-// Significant length of each product C_i of CL_i limbs whose operands had
-// nonzero top limbs: CL_i or CL_i - 1.
-struct TrimDesc {
-  const uint32_t *C;
-  unsigned long long CL;
-};
-__global__ void k_trim(const TrimDesc *d, uint32_t n, unsigned long long *len) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned long long CL = d[i].CL;
-  len[i] = CL - (CL > 1 && d[i].C[CL - 1] == 0 ? 1 : 0);
-}
-
 // R = X + Y for a batch of items: n = max(lx, ly) limbs of sum, then the
-// carry out as limb n (len = n + carry).  An item has n / ADD_TILE + 1 tiles
-// (the last one holds limb n) of ADD_TILE limbs; the carry
-// into a tile is found by a decoupled lookback over the tiles of the item,
-// with the carry maps {0,1} -> {0,1} kept in the {-1,0,1} map encoding of
-// the multiply's carry scan (fn_make / fn_compose).
+// carry out as limb n (len = n + carry).  X is a product of lx limbs whose
+// operands had nonzero top limbs, so its top limb alone may be zero: the
+// kernel takes lx - 1 then, and it also gives the significant length of a
+// second product q of ql limbs (the lengths would otherwise be a kernel and a
+// trip to the host of their own per tree level).  An item has max(lx, ly) /
+// ADD_TILE + 1 tiles of ADD_TILE limbs (the one that holds limb n is among
+// them; one beyond it may stay empty); the carry into a tile is found by a
+// decoupled lookback over the tiles of the item, with the carry maps {0,1} ->
+// {0,1} kept in the {-1,0,1} map encoding of the multiply's carry scan
+// (fn_make / fn_compose).  A status word carries all that it says, so it needs
+// no ordering of other memory.
 constexpr int ADD_NT = 256, ADD_PT = 8, ADD_TILE = ADD_NT * ADD_PT;
 
 struct AddDesc {
   const uint32_t *x;
   const uint32_t *y;
   uint32_t *r;
-  unsigned long long lx, ly, n;
+  const uint32_t *q;
+  unsigned long long lx, ly, ql;
   unsigned long long tile0;  // first tile of this item (batch-wide numbering)
 };
+
+// Limbs of a product of CL limbs without its top limb if that is zero.
+__device__ __forceinline__ unsigned long long product_len(const uint32_t *C, unsigned long long CL) {
+  return CL - (CL > 1 && C[CL - 1] == 0 ? 1 : 0);
+}
 
 struct AddParams {
   const AddDesc *items;
@@ -110,7 +109,7 @@ struct AddParams {
   unsigned long long tiles;
   unsigned int *counter;       // zeroed before launch
   uint32_t *status;            // one word per tile, zeroed before launch
-  unsigned long long *len;     // per item: n + carry out
+  unsigned long long *len;     // per item: n + carry out, length of q
   unsigned int *flags;         // bit 0: a lookback wait ran out
 };
 
@@ -131,6 +130,8 @@ __global__ void __launch_bounds__(ADD_NT) k_add(AddParams p) {
     }
     const AddDesc &it = p.items[lo];
     const unsigned long long tile = unit - it.tile0;
+    const unsigned long long lx = product_len(it.x, it.lx), n = lx > it.ly ? lx : it.ly;
+    if (tile == 0 && tid == 0) p.len[2 * lo + 1] = product_len(it.q, it.ql);
     const unsigned long long i0 = tile * ADD_TILE + (unsigned long long)tid * ADD_PT;
     uint32_t s[ADD_PT];
     unsigned c = 0;
@@ -138,11 +139,11 @@ __global__ void __launch_bounds__(ADD_NT) k_add(AddParams p) {
 #pragma unroll
     for (int q = 0; q < ADD_PT; q++) {
       const unsigned long long i = i0 + q;
-      const uint32_t xv = i < it.lx ? it.x[i] : 0u, yv = i < it.ly ? it.y[i] : 0u;
+      const uint32_t xv = i < lx ? it.x[i] : 0u, yv = i < it.ly ? it.y[i] : 0u;
       const unsigned long long v = (unsigned long long)xv + yv + c;
       s[q] = (uint32_t)v;
       c = (unsigned)(v >> 32);
-      if (i < it.n) ones = ones && s[q] == 0xffffffffu;
+      if (i < n) ones = ones && s[q] == 0xffffffffu;
     }
     // carry out of this thread's limbs given its carry in: c, or c | ones
     const int c0 = (int)c, c1 = (int)(c | (ones ? 1u : 0u));
@@ -153,17 +154,17 @@ __global__ void __launch_bounds__(ADD_NT) k_add(AddParams p) {
       cuda::atomic_ref<uint32_t, cuda::thread_scope_device> me(p.status[it.tile0 + tile]);
       int cin = 0;
       if (tile == 0) {
-        me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_release);
+        me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_relaxed);
       } else {
-        if (fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_release);
-        else me.store(ST_AGG | agg, cuda::memory_order_release);
+        if (fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, 0) + 1), cuda::memory_order_relaxed);
+        else me.store(ST_AGG | agg, cuda::memory_order_relaxed);
         uint32_t acc = FN_ID;
         long long prev = (long long)tile - 1;
         int spins = 0;
         bool timed_out = false;
         for (;;) {
           cuda::atomic_ref<uint32_t, cuda::thread_scope_device> st(p.status[it.tile0 + prev]);
-          const uint32_t v = st.load(cuda::memory_order_acquire);
+          const uint32_t v = st.load(cuda::memory_order_relaxed);
           if (v & ST_INC) {
             cin = fn_apply(acc, (int)(v & 3u) - 1);
             break;
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(ADD_NT) k_add(AddParams p) {
           atomicOr(p.flags, 1u);
           cin = 0;
         }
-        if (!fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, cin) + 1), cuda::memory_order_release);
+        if (!fn_is_const(agg)) me.store(ST_INC | (uint32_t)(fn_apply(agg, cin) + 1), cuda::memory_order_relaxed);
       }
       s_cin = cin;
     }
@@ -194,13 +195,13 @@ __global__ void __launch_bounds__(ADD_NT) k_add(AddParams p) {
       const unsigned long long i = i0 + q;
       const unsigned long long v = (unsigned long long)s[q] + cc;
       cc = (unsigned)(v >> 32);
-      if (i < it.n) it.r[i] = (uint32_t)v;
-      else if (i == it.n) { top = (uint32_t)v; has_top = true; }
+      if (i < n) it.r[i] = (uint32_t)v;
+      else if (i == n) { top = (uint32_t)v; has_top = true; }
     }
     // limb n (inside the item's last tile) is the carry out of limb n-1
     if (has_top) {
-      it.r[it.n] = top;
-      p.len[lo] = it.n + top;
+      it.r[n] = top;
+      p.len[2 * lo] = n + top;
     }
     __syncthreads();
   }

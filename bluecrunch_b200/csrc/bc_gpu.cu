@@ -2472,68 +2472,48 @@ int e_series_locked(uint32_t a, uint32_t b, uint32_t **hP, size_t *PL, uint32_t 
     const double dm = secs(tl0);
     t_mul += dm;
     tl0 = now();
-    // significant lengths of the products, then the additions
-    std::vector<TrimDesc> td(2 * np);
-    for (size_t i = 0; i < 2 * np; i++) td[i] = {md[i].C, md[i].CL};
+    // the additions, with the significant lengths of both products (see k_add)
     std::vector<AddDesc> ad(np);
-    unsigned long long tiles = 0;  // bound from the untrimmed lengths; sizes the status words
+    unsigned long long tiles = 0;
     for (size_t i = 0; i < np; i++) {
-      const unsigned long long n = std::max<unsigned long long>(nT[i], P[2 * i + 1].len);
-      ad[i] = {nb + offT[i], P[2 * i + 1].p, nb + offP[i], nT[i], P[2 * i + 1].len, n, 0};
-      tiles += n / ADD_TILE + 1;
+      ad[i] = {nb + offT[i], P[2 * i + 1].p, nb + offP[i], nb + offQ[i], nT[i], P[2 * i + 1].len, nQ[i], tiles};
+      tiles += std::max<unsigned long long>(nT[i], P[2 * i + 1].len) / ADD_TILE + 1;
     }
-    // scratch: trim descs, product lengths, add descs, status, counter+flags, add lengths
-    const size_t o_td = 0, o_tl = align256(o_td + td.size() * sizeof(TrimDesc));
-    const size_t o_ad = align256(o_tl + 2 * np * 8), o_st = align256(o_ad + np * sizeof(AddDesc));
-    const size_t o_ctr = align256(o_st + tiles * 4), o_al = o_ctr + 256, o_end = align256(o_al + np * 8);
+    // scratch: descriptors, status, counter, then lengths and flags (read back in one copy)
+    const size_t o_ad = 0, o_st = align256(np * sizeof(AddDesc)), o_ctr = align256(o_st + tiles * 4);
+    const size_t o_al = o_ctr + 256, o_fl = o_al + np * 16, o_end = align256(o_fl + 8);
     DevBuf meta;
     if ((r = meta.alloc(o_end))) return r;
     char *mb = (char *)meta.p;
-    CK(cudaMemcpyAsync(mb + o_td, td.data(), td.size() * sizeof(TrimDesc), cudaMemcpyHostToDevice, g.stream));
-    k_trim<<<(unsigned)((2 * np + 255) / 256), 256, 0, g.stream>>>((const TrimDesc *)(mb + o_td), (uint32_t)(2 * np),
-                                                                 (unsigned long long *)(mb + o_tl));
-    CK(cudaGetLastError());
-    std::vector<unsigned long long> tl(2 * np);
-    CK(cudaMemcpyAsync(tl.data(), mb + o_tl, tl.size() * 8, cudaMemcpyDeviceToHost, g.stream));
-    CK(cudaStreamSynchronize(g.stream));
-    tiles = 0;
-    for (size_t i = 0; i < np; i++) {
-      ad[i].lx = tl[2 * i];
-      ad[i].n = std::max<unsigned long long>(ad[i].lx, ad[i].ly);
-      ad[i].tile0 = tiles;
-      tiles += ad[i].n / ADD_TILE + 1;
-    }
     CK(cudaMemcpyAsync(mb + o_ad, ad.data(), ad.size() * sizeof(AddDesc), cudaMemcpyHostToDevice, g.stream));
-    CK(cudaMemsetAsync(mb + o_st, 0, o_al - o_st, g.stream));
+    CK(cudaMemsetAsync(mb + o_st, 0, o_end - o_st, g.stream));
     AddParams ap;
     ap.items = (const AddDesc *)(mb + o_ad);
     ap.nitems = (int)np;
     ap.tiles = tiles;
     ap.counter = (unsigned int *)(mb + o_ctr);
-    ap.flags = (unsigned int *)(mb + o_ctr + 128);
+    ap.flags = (unsigned int *)(mb + o_fl);
     ap.status = (uint32_t *)(mb + o_st);
     ap.len = (unsigned long long *)(mb + o_al);
     const unsigned grid = (unsigned)std::min<unsigned long long>(tiles, (unsigned long long)g.sm_count * 4);
     k_add<<<grid, ADD_NT, 0, g.stream>>>(ap);
     CK(cudaGetLastError());
-    std::vector<unsigned long long> al(np);
-    unsigned int aflags = 0;
-    CK(cudaMemcpyAsync(al.data(), ap.len, np * 8, cudaMemcpyDeviceToHost, g.stream));
-    CK(cudaMemcpyAsync(&aflags, ap.flags, 4, cudaMemcpyDeviceToHost, g.stream));
+    std::vector<unsigned long long> al(2 * np + 1);  // the last one: the flags
+    CK(cudaMemcpyAsync(al.data(), ap.len, np * 16 + 8, cudaMemcpyDeviceToHost, g.stream));
     if (odd) {
       CK(cudaMemcpyAsync(nb + offOddP, P[c - 1].p, P[c - 1].len * 4, cudaMemcpyDeviceToDevice, g.stream));
       CK(cudaMemcpyAsync(nb + offOddQ, Q[c - 1].p, Q[c - 1].len * 4, cudaMemcpyDeviceToDevice, g.stream));
     }
     CK(cudaStreamSynchronize(g.stream));
-    if (aflags) return fail(BC_ERR_TIMEOUT);
+    if (al[2 * np]) return fail(BC_ERR_TIMEOUT);
     const double da = secs(tl0);
     t_add += da;
     if (stats && (dm + da > 0.05 || np < 4))
       fprintf(stderr, "      series level: %zu nodes, products %.3f s, lengths and sums %.3f s\n", np, dm, da);
     std::vector<DevNum> P2(np + odd), Q2(np + odd);
     for (size_t i = 0; i < np; i++) {
-      P2[i] = {nb + offP[i], (size_t)al[i]};
-      Q2[i] = {nb + offQ[i], (size_t)tl[2 * i + 1]};
+      P2[i] = {nb + offP[i], (size_t)al[2 * i]};
+      Q2[i] = {nb + offQ[i], (size_t)al[2 * i + 1]};
     }
     if (odd) {
       P2[np] = {nb + offOddP, P[c - 1].len};
