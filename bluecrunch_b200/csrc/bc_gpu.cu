@@ -506,11 +506,10 @@ KInfo small_info() {
   return {(const void *)k_small<M, SQ>, M / PTS, TileSmem<M, 1>::elems * sizeof(double2), "small", SIG_P};
 }
 
-template <int L>
-KInfo outer_fwd16_info(int parts) {
-  using T = Pass16<L>;
-  KInfo k{parts == 1 ? (const void *)k3_outer_fwd<L, 1> : (const void *)k3_outer_fwd<L, 2>, T::NT, T::SMEM_FWD(parts),
-          "outer_fwd", SIG_P};
+template <int L, int PARTS>
+KInfo outer_fwd16_info() {
+  using T = Fwd16<L, PARTS>;
+  KInfo k{(const void *)k3_outer_fwd<L, PARTS>, T::NT, T::SMEM, "outer_fwd", SIG_P};
   k.pts = P16;
   return k;
 }
@@ -526,9 +525,9 @@ KInfo outer_inv16_info() {
 KInfo get_outer(int L, bool inv, int parts = 2) {
   if (g.pass16) {
     switch (L) {
-      case 64: return inv ? outer_inv16_info<64>() : outer_fwd16_info<64>(parts);
-      case 128: return inv ? outer_inv16_info<128>() : outer_fwd16_info<128>(parts);
-      case 256: return inv ? outer_inv16_info<256>() : outer_fwd16_info<256>(parts);
+      case 64: return inv ? outer_inv16_info<64>() : parts == 1 ? outer_fwd16_info<64, 1>() : outer_fwd16_info<64, 2>();
+      case 128: return inv ? outer_inv16_info<128>() : parts == 1 ? outer_fwd16_info<128, 1>() : outer_fwd16_info<128, 2>();
+      case 256: return inv ? outer_inv16_info<256>() : parts == 1 ? outer_fwd16_info<256, 1>() : outer_fwd16_info<256, 2>();
     }
   }
   switch (L) {
@@ -729,8 +728,9 @@ bool shape_launch_ok(const Shape &s, bool sq) {
     const KInfo kmf = get_mid(s.L2, false), kmi = get_mid(s.L2, true);
     if (!kmf.fn || !kmi.fn || kmf.smem > kMaxSmemPerCta || kmi.smem > kMaxSmemPerCta) return false;
   }
-  const int W1 = ko.threads / (s.L1 / ko.pts);
-  if (S1 % W1 || W1 % 8 || ki.threads / (s.L1 / ki.pts) != W1) return false;
+  const int WF = ko.threads / (s.L1 / ko.pts), W1 = ki.threads / (s.L1 / ki.pts);
+  if (S1 % W1 || W1 % 8 || S1 % WF || WF % 8) return false;
+  if (get_outer(s.L1, false, 1).smem > kMaxSmemPerCta) return false;
   if ((size_t)(W1 / 8) * ki.parts * 128 * ki.box != ki.unit_bytes || (size_t)ki.box * ki.parts != (size_t)s.L1)
     return false;
   const int NR = kr.rows ? kr.rows : (kr.warp_rows ? 1 : kr.threads / ((int)Lr / PTS));
@@ -784,7 +784,7 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
   }
   const cuuint64_t M16 = (cuuint64_t)s.M * 16, S1 = (cuuint64_t)params.S1, Lr = (cuuint64_t)params.Lr;
   KInfo ko = get_outer(s.L1, false, params.parts == 1 ? 1 : 2), ki = get_outer(s.L1, true);
-  const int W1 = ko.threads / (s.L1 / ko.pts);
+  const int WF = ko.threads / (s.L1 / ko.pts), W1 = ki.threads / (s.L1 / ki.pts);  // tile columns, forward and inverse
   ClassParams p = params;
   p.fd_outer = FastDiv((uint32_t)(S1 / W1));
   p.fd_rows = FastDiv((uint32_t)(s.M / Lr));
@@ -792,6 +792,7 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
     const KInfo km = get_mid(s.L2, false);
     p.fd_mid = FastDiv((uint32_t)(Lr / (km.threads / (s.L2 / km.pts))));
     p.fd_op = FastDiv((uint32_t)s.L1 * p.fd_mid.d);
+  p.fd_fwd = FastDiv((uint32_t)(S1 / WF));
   }
   // forward operands: every item's A, then the B slab's slots (items sharing
   // a B share a slot)
@@ -801,10 +802,10 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
     ClassParams pa = p, pb = p;
     pa.fwd_ops = 1;
     pb.fwd_ops = 2;
-    if ((r = launch(ko, n * (long long)(S1 / W1), pa, nl, stream, timed))) return r;
+    if ((r = launch(ko, n * (long long)(S1 / WF), pa, nl, stream, timed))) return r;
     CK(cudaStreamWaitEvent(stream, b_ready, 0));
-    if ((r = launch(ko, nb * (long long)(S1 / W1), pb, nl, stream, timed))) return r;
-  } else if ((r = launch(ko, (n + nb) * (long long)(S1 / W1), p, nl, stream, timed))) {
+    if ((r = launch(ko, nb * (long long)(S1 / WF), pb, nl, stream, timed))) return r;
+  } else if ((r = launch(ko, (n + nb) * (long long)(S1 / WF), p, nl, stream, timed))) {
     return r;
   }
   pdl = pdl_ok;

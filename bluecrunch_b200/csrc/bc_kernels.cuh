@@ -86,10 +86,11 @@ struct ClassParams {
   // count of finished column items, then of finished row items; zeroed
   // before launch.  Null: the middle runs as separate passes.
   unsigned int *blkdone;
-  // divisions of unit numbers: by the column tiles of the outer passes, the
+  // divisions of unit numbers: by the column tiles of the outer passes (forward,
+  // inverse), the
   // units of one operand and the column tiles of a block in the middle passes,
   // and the rows of an item (launch_class fills them in)
-  FastDiv fd_outer, fd_op, fd_mid, fd_rows;
+  FastDiv fd_fwd, fd_outer, fd_op, fd_mid, fd_rows;
   double2 *slabA, *slabB;          // the class's A and B slabs (item i at slab + i*slab_elems)
   unsigned long long slab_elems;
   // A product alone in its call: its descriptor comes with the first kernel's

@@ -107,16 +107,9 @@ template <int L> struct Pass16 {
   static_assert(L == 64 || L == 128 || L == 256, "16-point passes cover L1 = 64, 128, 256");
   // twelve warps per SM (at most 170 registers per thread)
   static constexpr int MINB = 384 / NT;
-  // the forward pass of operands without digits at M or above (no imaginary
-  // parts, half the limb stage): sixteen (128 registers; L = 64 would spill)
-  static constexpr int MINB_FWD(int parts) { return parts == 1 && L > 64 ? 512 / NT : MINB; }
   // dynamic shared memory
   static constexpr size_t TWB = (size_t)L * 16;  // block16 twiddles
   static constexpr size_t SMEM_INV = 2 * (size_t)L * W * 16 + TWB + (size_t)L * 16 + 2 * 38 * 16 + 1024;
-  static constexpr size_t SMEM_FWD(int parts) {
-    return (size_t)L * W * 16 + (size_t)PackTile<L>::STAGE_WORDS / 2 * parts * 4 + TWB + (size_t)L * 16 + 2 * 38 * 16 +
-           1024;
-  }
 };
 
 // Outer-pass twiddles e^{-2 pi i col (4 k1 - 1)/(4M)} of one thread, for
@@ -195,24 +188,36 @@ __device__ __forceinline__ OuterRun16 outer_run16(const double2 *fac, const ColT
 // next unit's words are copied (cp.async) as soon as this unit's digits are
 // cut, and land while this unit is transformed and stored.
 // PARTS: 1 when no operand of the class has digits at M or above (products of
-// operands of about one length), so the limb stage holds one part and four
-// CTAs of 128 threads fit an SM instead of three: 0.360 ms against 0.380 at 2^25
-// points.
+// operands of about one length): the limb stage then holds one part, and
+// sixteen warps of 128 registers fit an SM instead of twelve (L = 64 would
+// spill): 0.380 -> 0.360 ms at 2^25 points (L = 256).  Columns of up to 128
+// points take tiles of 16 columns, 256-byte segments and fewer limb copies per
+// digit (whole 2^21-point product 0.112 -> 0.108 ms); at 256 points a CTA of
+// 256 threads lost more than that (2^23 points 0.394 -> 0.405 ms).
+template <int L, int PARTS> struct Fwd16 {
+  static constexpr int W = L < 256 ? 16 : 8;
+  static constexpr int R = L / P16, NT = R * W;
+  static constexpr int MINB = (PARTS == 1 && L > 64 ? 512 : 384) / NT;
+  using Stage = PackTile<L, W>;
+  static constexpr int STAGE_WORDS = Stage::STAGE_WORDS / 2 * PARTS;
+  static constexpr size_t SMEM = (size_t)L * W * 16 + (size_t)STAGE_WORDS * 4 + 2 * (size_t)L * 16 +
+                                 2 * TILE_TW_N * 16 + 1024;
+};
+
 template <int L, int PARTS>
-__global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB_FWD(PARTS)) k3_outer_fwd(const __grid_constant__ ClassParams p) {
+__global__ void __launch_bounds__(Fwd16<L, PARTS>::NT, Fwd16<L, PARTS>::MINB) k3_outer_fwd(const __grid_constant__ ClassParams p) {
   pdl_trigger();  // the first pass of a class: launched normally, lets the next one start early
-  using T = Pass16<L>;
-  using K = PackTile<L>;
+  using T = Fwd16<L, PARTS>;
+  using K = typename T::Stage;
   constexpr int W = T::W, R = T::R, NT = T::NT;
-  static_assert(K::W == W, "pack tile geometry");
   extern __shared__ unsigned char smraw[];
   double2 *tile = align1024(smraw);
   uint32_t *stg = reinterpret_cast<uint32_t *>(tile + L * W);  // one stage: L segments per part
-  double2 *twS = reinterpret_cast<double2 *>(stg + K::STAGE_WORDS / 2 * PARTS);
+  double2 *twS = reinterpret_cast<double2 *>(stg + T::STAGE_WORDS);
   double2 *pwS = twS + L;
   double2 *fac = pwS + L;  // tile factors of a unit, of the units in turn at fac + par * TILE_TW_N
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
-  const int tiles = (int)p.fd_outer.d;
+  const int tiles = (int)p.fd_fwd.d;
   const unsigned nA = fwd_units_a(p, (unsigned)tiles);
   const unsigned total = nA + fwd_units_b(p, (unsigned)tiles);  // far below 2^32
   // limb staging: as k2_outer_fwd (every row segment of a tile shares one
@@ -223,7 +228,7 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB_FWD(PARTS)) k3_
   // the unit's limb words and, to the set `par`, its tile factors (the threads
   // still at the unit before read the other set)
   auto stage_copy = [&](unsigned u, int par) {
-    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_fwd, (unsigned)tiles);
     const int tl = (int)f.rest;
     tile_tw16<R, W>(fac + par * TILE_TW_N, tl, p.tw4M, p.M);
     const FwdOperand it = fwd_operand(p, f.item, f.op);
@@ -235,8 +240,11 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB_FWD(PARTS)) k3_
     const int wbase = ((tl * W * b) >> 5) - 1 - seg_shift(tl, b, al16);
     const int parts = PARTS == 2 && it.nd > (unsigned)p.M ? 2 : 1;
     if (al16) {
+      // the chunks up to the last digit's last bit (the second word that its
+      // cut reads may lie beyond: those bits are masked away)
       constexpr int CH = K::SEGW4 / 4;
       const int NCH = parts * L * CH;
+      const int need = ((32 * (1 + seg_shift(tl, b, true)) + ((tl * W * b) & 31) + W * b - 1) >> 5) / 4 + 1;
       for (int idx = tid; idx < NCH; idx += NT) {
         const int segi = idx / CH, k = idx - segi * CH;
         const int part = segi >= L, row = segi - (part ? L : 0);
@@ -244,7 +252,7 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB_FWD(PARTS)) k3_
         int nv = XL - w;
         nv = nv < 0 ? 0 : (nv > 4 ? 4 : nv);
         if (w < 0) nv = 0;
-        cp_async16(stg + segi * K::SEGW4 + 4 * k, X + (nv ? w : 0), nv * 4);
+        if (k < need) cp_async16(stg + segi * K::SEGW4 + 4 * k, X + (nv ? w : 0), nv * 4);
       }
     } else {
       for (int idx = tid; idx < parts * (K::STAGE_WORDS / 2); idx += NT) {
@@ -265,7 +273,7 @@ __global__ void __launch_bounds__(Pass16<L>::NT, Pass16<L>::MINB_FWD(PARTS)) k3_
   table_to_smem<L, NT>(pwS, p.pw_fwd);
   const ColTw16 ct = col_tw16<R>(s, t, p.tw4M, p.M);
   for (int par = 0; u < total; u += gridDim.x, par ^= 1) {
-    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_fwd, (unsigned)tiles);
     const int tl = (int)f.rest;
     const FwdOperand it = fwd_operand(p, f.item, f.op);
     const int col = tl * W + s;

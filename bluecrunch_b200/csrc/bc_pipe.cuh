@@ -512,8 +512,8 @@ __global__ void __launch_bounds__(RowTile<L>::NT, RowTile<L>::MINB)
 // Units: (item, operand, column tile).  The limb words behind each tile row
 // (real and imaginary digit runs) are staged with cp.async one unit ahead;
 // digits are cut from shared memory.
-template <int L> struct PackTile {
-  static constexpr int W = PassTile<L>::W;
+template <int L, int TW = PassTile<L>::W> struct PackTile {
+  static constexpr int W = TW;  // columns of a tile
   // words per staged row segment for widths up to 24 bits: the segment starts
   // one word below the first digit's word and must hold the 64-bit window of
   // the last digit (start offset < 64 bits, last window ends below 24W + 95)
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
   double2 *twS = reinterpret_cast<double2 *>(stg + 2 * K::STAGE_WORDS);
   double2 *pwS = twS + tw_entries<L>();
   const int tid = threadIdx.x, s = tid % W, t = tid / W;
-  const int tiles = (int)p.fd_outer.d;
+  const int tiles = (int)p.fd_fwd.d;
   const unsigned nA = fwd_units_a(p, (unsigned)tiles);
   const unsigned total = nA + fwd_units_b(p, (unsigned)tiles);  // far below 2^32
   // Row segment (n1, part) of tile tl starts one word below the word of digit
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
     return al16 ? (int)((((long long)tl * W * b >> 5) - 1) & 3) : 0;
   };
   auto stage_copy = [&](unsigned u, int st) {
-    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_fwd, (unsigned)tiles);
     const int tl = (int)f.rest;
     const FwdOperand it = fwd_operand(p, f.item, f.op);
     const uint32_t *X = it.X;
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
-    const FwdUnit f = fwd_unit(p, u, nA, p.fd_outer, (unsigned)tiles);
+    const FwdUnit f = fwd_unit(p, u, nA, p.fd_fwd, (unsigned)tiles);
     const int tl = (int)f.rest;
     const FwdOperand it = fwd_operand(p, f.item, f.op);
     const unsigned nd = it.nd;
