@@ -57,6 +57,12 @@ constexpr int kRowLens[] = {128, 192, 256, 320, 384, 512, 640, 768, 1024, 1280, 
 constexpr int kSmallLens[] = {256, 512, 768, 1024, 1280, 1536, 2048, 2560, 3072, 4096, 5120};
 constexpr int kOuterLens[] = {64, 128, 256, 512};
 constexpr size_t kMaxM = size_t(1) << 30;
+// Two levels up to this length, three above: two levels of 2^20 points and
+// more need rows of 2,560 to 4,096 points, which only the general row kernel
+// has.  Full-size products, two against three levels (ms): 2^19 0.067 / 0.076,
+// 3*2^18 0.089 / 0.085, 2^20 0.092 / 0.098, 5*2^18 0.129 / 0.113, 3*2^19
+// 0.149 / 0.121, 2^21 0.155 / 0.136.
+constexpr size_t kTwoLevelPoints = size_t(1) << 20;
 
 bool is_row_len(size_t L) {
   for (int x : kRowLens) if ((size_t)x == L) return true;
@@ -76,7 +82,7 @@ bool shape_default(size_t M, Shape &s) {
     return false;
   }
   for (int L1 : kOuterLens) {
-    if (M % L1) continue;
+    if (M % L1 || M > kTwoLevelPoints) continue;
     const size_t Lr = M / L1;
     if (is_row_len(Lr) && pow2part(Lr) >= (size_t)pass_tile_w(L1)) {
       s.M = (int)M; s.L1 = L1; s.L2 = 1; s.Lr = (int)Lr; s.levels = 2; return true;
@@ -84,7 +90,7 @@ bool shape_default(size_t M, Shape &s) {
   }
   // three levels: rows of about 1024 points keep the fused row pass free of
   // spills with two rows per CTA; longer rows only when the outer passes run out
-  static const int kRowPref[] = {1024, 768, 1536, 512, 2048, 3072, 4096, 1280, 640, 2560};
+  static const int kRowPref[] = {1024, 768, 1536, 512, 2048, 3072, 4096, 1280, 640, 2560, 384, 320, 256, 192, 128};
   for (int Lri : kRowPref) {
     const size_t Lr = (size_t)Lri;
     if (M % Lr) continue;
@@ -574,7 +580,7 @@ KInfo get_rows(int L, bool sq) {
   }
   if (g.rows_warp) {
     switch (L) {
-      ROW2CASE(128) ROW2CASE(192) ROW2CASE(256) ROW2CASE(320) ROW2CASE(384)
+      ROW2CASE(128) ROW2CASE(192) ROW2CASE(256) ROW2CASE(320) ROW2CASE(384) ROW2CASE(640) ROW2CASE(768)
     }
   }
   switch (L) {
@@ -786,13 +792,13 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
   KInfo ko = get_outer(s.L1, false, params.parts == 1 ? 1 : 2), ki = get_outer(s.L1, true);
   const int WF = ko.threads / (s.L1 / ko.pts), W1 = ki.threads / (s.L1 / ki.pts);  // tile columns, forward and inverse
   ClassParams p = params;
+  p.fd_fwd = FastDiv((uint32_t)(S1 / WF));
   p.fd_outer = FastDiv((uint32_t)(S1 / W1));
   p.fd_rows = FastDiv((uint32_t)(s.M / Lr));
   if (s.levels == 3) {
     const KInfo km = get_mid(s.L2, false);
     p.fd_mid = FastDiv((uint32_t)(Lr / (km.threads / (s.L2 / km.pts))));
     p.fd_op = FastDiv((uint32_t)s.L1 * p.fd_mid.d);
-  p.fd_fwd = FastDiv((uint32_t)(S1 / WF));
   }
   // forward operands: every item's A, then the B slab's slots (items sharing
   // a B share a slot)

@@ -65,22 +65,24 @@ __device__ __forceinline__ void dft_regs(double2 (&x)[N]) {
   else if constexpr (N == 12) dft_coprime<3, 4, INV>(x);
   else if constexpr (N == 16) dft16<INV>(x);
   else if constexpr (N == 20) dft_coprime<5, 4, INV>(x);
-  else dft_coprime<3, 8, INV>(x);
-  static_assert(N == 8 || N == 12 || N == 16 || N == 20 || N == 24, "lengths in registers");
+  else if constexpr (N == 24) dft_coprime<3, 8, INV>(x);
+  else dft32<INV>(x);
+  static_assert(N == 8 || N == 12 || N == 16 || N == 20 || N == 24 || N == 32, "lengths in registers");
 }
 
 template <int L> struct Rows2 {
-  static constexpr int P2 = L == 128 ? 8 : (L == 192 ? 12 : 16);
+  static constexpr int P2 = L == 128 ? 8 : (L == 192 ? 12 : (L <= 384 ? 16 : 32));
   static constexpr int P1 = L / P2;
   static constexpr int TR = P1 > P2 ? P1 : P2;      // threads per row
-  static constexpr int NR = 8;                      // rows per unit
+  static constexpr int NR = L == 640 ? 4 : 8;       // rows per unit
   static constexpr int NT = NR * TR;
   static constexpr bool WARP = 32 % TR == 0;        // rows private to a warp
   static constexpr int PITCH = P2 | 1;
   static constexpr int ROW = (P1 * PITCH > L ? P1 * PITCH : L);  // entries of a row's buffer
-  // ten or twelve warps per SM, at most 168 registers; B's spectrum stays in
-  // registers where that leaves room, else in B's buffer
-  static constexpr int MINB = NT == 128 ? 3 : 2;
+  // ten or twelve warps per SM, at most 168 registers (640 and 768 points:
+  // eight, 255); B's spectrum stays in registers where that leaves room, else
+  // in B's buffer
+  static constexpr int MINB = L == 768 ? 1 : (L == 640 || NT != 128 ? 2 : 3);
   static constexpr bool PARK = L >= 320;
   static constexpr size_t SMEM = (size_t)(2 * NR * ROW + L) * 16;
   static_assert(NT % 32 == 0, "whole warps");

@@ -1,4 +1,4 @@
-"""GPU: row passes of 128, 192, 256, 320 and 384 points (k5_rows,
+"""GPU: row passes of 128, 192, 256, 320, 384, 640 and 768 points (k5_rows,
 csrc/bc_rows2.cuh) inside two- and three-level transforms, against exact
 products: full lengths, operands longer than half of the transform, squares, and
 a batch whose items share a transform length (several items, B shared)."""
@@ -11,10 +11,10 @@ from conftest import limbs
 pytestmark = pytest.mark.gpu
 
 # (M, L1, L2, Lr): every row length with two levels, and with three
-SHAPES = [(64 * r, 64, 1, r) for r in (128, 192, 256, 320, 384)] + \
-         [(512 * r, 512, 1, r) for r in (128, 192, 256, 320, 384)] + \
+SHAPES = [(64 * r, 64, 1, r) for r in (128, 192, 256, 320, 384, 640, 768)] + \
+         [(512 * r, 512, 1, r) for r in (128, 192, 256, 320, 384, 640, 768)] + \
          [(64 * 64 * 256, 64, 64, 256), (128 * 64 * 320, 128, 64, 320), (64 * 128 * 384, 64, 128, 384),
-          (128 * 128 * 192, 128, 128, 192), (256 * 128 * 128, 256, 128, 128)]
+          (128 * 128 * 192, 128, 128, 192), (256 * 128 * 128, 256, 128, 128), (64 * 64 * 640, 64, 64, 640), (64 * 64 * 768, 64, 64, 768)]
 
 
 @pytest.mark.parametrize("M,L1,L2,Lr", SHAPES)
