@@ -512,10 +512,10 @@ KInfo small_info() {
   return {(const void *)k_small<M, SQ>, M / PTS, TileSmem<M, 1>::elems * sizeof(double2), "small", SIG_P};
 }
 
-template <int L, int PARTS>
+template <int L, int PARTS, int TW>
 KInfo outer_fwd16_info() {
-  using T = Fwd16<L, PARTS>;
-  KInfo k{(const void *)k3_outer_fwd<L, PARTS>, T::NT, T::SMEM, "outer_fwd", SIG_P};
+  using T = Fwd16<L, PARTS, TW>;
+  KInfo k{(const void *)k3_outer_fwd<L, PARTS, TW>, T::NT, T::SMEM, "outer_fwd", SIG_P};
   k.pts = P16;
   return k;
 }
@@ -528,12 +528,20 @@ KInfo outer_inv16_info() {
   return k;
 }
 
-KInfo get_outer(int L, bool inv, int parts = 2) {
+// parts, wide: the forms of the forward pass (see Fwd16).
+KInfo get_outer(int L, bool inv, int parts = 2, bool wide = true) {
   if (g.pass16) {
     switch (L) {
-      case 64: return inv ? outer_inv16_info<64>() : parts == 1 ? outer_fwd16_info<64, 1>() : outer_fwd16_info<64, 2>();
-      case 128: return inv ? outer_inv16_info<128>() : parts == 1 ? outer_fwd16_info<128, 1>() : outer_fwd16_info<128, 2>();
-      case 256: return inv ? outer_inv16_info<256>() : parts == 1 ? outer_fwd16_info<256, 1>() : outer_fwd16_info<256, 2>();
+      case 64:
+        if (inv) return outer_inv16_info<64>();
+        return parts == 1 ? outer_fwd16_info<64, 1, 16>() : outer_fwd16_info<64, 2, 16>();
+      case 128:
+        if (inv) return outer_inv16_info<128>();
+        if (wide) return parts == 1 ? outer_fwd16_info<128, 1, 16>() : outer_fwd16_info<128, 2, 16>();
+        return parts == 1 ? outer_fwd16_info<128, 1, 8>() : outer_fwd16_info<128, 2, 8>();
+      case 256:
+        if (inv) return outer_inv16_info<256>();
+        return parts == 1 ? outer_fwd16_info<256, 1, 8>() : outer_fwd16_info<256, 2, 8>();
     }
   }
   switch (L) {
@@ -789,7 +797,9 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
     return launch(n * kc.cluster <= 2 * g.sm_count ? kc : get_small(s.M, sq), n, params, nl, stream, timed);
   }
   const cuuint64_t M16 = (cuuint64_t)s.M * 16, S1 = (cuuint64_t)params.S1, Lr = (cuuint64_t)params.Lr;
-  KInfo ko = get_outer(s.L1, false, params.parts == 1 ? 1 : 2), ki = get_outer(s.L1, true);
+  const long long nfwd = n + (sq ? 0 : (long long)params.nb);  // forward operands
+  const bool wide = nfwd * (long long)(S1 / 16) >= 2 * (long long)g.sm_count;
+  KInfo ko = get_outer(s.L1, false, params.parts == 1 ? 1 : 2, wide), ki = get_outer(s.L1, true);
   const int WF = ko.threads / (s.L1 / ko.pts), W1 = ki.threads / (s.L1 / ki.pts);  // tile columns, forward and inverse
   ClassParams p = params;
   p.fd_fwd = FastDiv((uint32_t)(S1 / WF));

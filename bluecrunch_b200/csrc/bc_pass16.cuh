@@ -190,12 +190,14 @@ __device__ __forceinline__ OuterRun16 outer_run16(const double2 *fac, const ColT
 // PARTS: 1 when no operand of the class has digits at M or above (products of
 // operands of about one length): the limb stage then holds one part, and
 // sixteen warps of 128 registers fit an SM instead of twelve (L = 64 would
-// spill): 0.380 -> 0.360 ms at 2^25 points (L = 256).  Columns of up to 128
-// points take tiles of 16 columns, 256-byte segments and fewer limb copies per
-// digit (whole 2^21-point product 0.112 -> 0.108 ms); at 256 points a CTA of
-// 256 threads lost more than that (2^23 points 0.394 -> 0.405 ms).
-template <int L, int PARTS> struct Fwd16 {
-  static constexpr int W = L < 256 ? 16 : 8;
+// spill): 0.380 -> 0.360 ms at 2^25 points (L = 256).
+// TW: columns of a tile.  At L = 128, 16 where that still gives every SM two
+// units (256-byte segments, fewer limb copies per digit: whole 2^21-point
+// product 0.112 -> 0.108 ms), else 8 (2^15 points 0.045 -> 0.043 ms a call).
+// At L = 256 always 8: a CTA of 256 threads lost more than it gained (2^23
+// points 0.394 -> 0.405 ms).
+template <int L, int PARTS, int TW> struct Fwd16 {
+  static constexpr int W = TW;
   static constexpr int R = L / P16, NT = R * W;
   static constexpr int MINB = (PARTS == 1 && L > 64 ? 512 : 384) / NT;
   using Stage = PackTile<L, W>;
@@ -204,10 +206,11 @@ template <int L, int PARTS> struct Fwd16 {
                                  2 * TILE_TW_N * 16 + 1024;
 };
 
-template <int L, int PARTS>
-__global__ void __launch_bounds__(Fwd16<L, PARTS>::NT, Fwd16<L, PARTS>::MINB) k3_outer_fwd(const __grid_constant__ ClassParams p) {
+template <int L, int PARTS, int TW>
+__global__ void __launch_bounds__(Fwd16<L, PARTS, TW>::NT, Fwd16<L, PARTS, TW>::MINB)
+    k3_outer_fwd(const __grid_constant__ ClassParams p) {
   pdl_trigger();  // the first pass of a class: launched normally, lets the next one start early
-  using T = Fwd16<L, PARTS>;
+  using T = Fwd16<L, PARTS, TW>;
   using K = typename T::Stage;
   constexpr int W = T::W, R = T::R, NT = T::NT;
   extern __shared__ unsigned char smraw[];
