@@ -166,6 +166,10 @@ struct Ctx {
   bool pdl = true;
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t gexec = nullptr;
+  // kernels of the capture in progress and of gexec, in launch order, a null
+  // entry before each class's (launch_graph)
+  std::vector<const void *> cap_fns, gexec_fns;
+  bool capturing = false;
   std::vector<std::pair<const char *, double>> ktimes;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<cudaEvent_t> kev;
@@ -678,6 +682,7 @@ int launch(const KInfo &k, long long units, const ClassParams &p, size_t *nlaunc
     CK(cudaLaunchKernel(k.fn, dim3(grid), dim3(k.threads), args, k.smem, stream));
   }
   (*nlaunch)++;
+  if (g.capturing) g.cap_fns.push_back(k.fn);
   if (timed && g.time_kernels) {
     cudaEvent_t e;
     if (!g.kev_pool.empty()) {
@@ -1186,6 +1191,7 @@ constexpr size_t kPdlMaxPoints = size_t(1) << 27;
 struct CaptureGuard {
   cudaStream_t s = nullptr;
   ~CaptureGuard() {
+    g.capturing = false;
     if (!s) return;
     cudaGraph_t gr = nullptr;
     cudaStreamEndCapture(s, &gr);
@@ -1194,16 +1200,19 @@ struct CaptureGuard {
   }
 };
 
-// The captured graph replaces the kept executable graph's contents when its
-// launch structure is the same (cudaGraphExecUpdate), else it is instantiated
-// anew; then one cudaGraphLaunch on the library stream runs every class.
+// The captured graph replaces the kept executable graph's contents when it
+// launches the same kernels in the same order (cudaGraphExecUpdate: addresses
+// and grids change), else it is instantiated anew; then one cudaGraphLaunch on
+// the library stream runs every class.  A node is never given another kernel:
+// the small products' kernels have clusters or not, and an update from one to
+// the other was accepted, but products of that batch did not run.
 int launch_graph(cudaGraph_t gr, bc_batch_stats *st) {
   size_t nodes = 0;
   cudaGraphGetNodes(gr, nullptr, &nodes);
   bool updated = false;
   if (g.gexec) {
     cudaGraphExecUpdateResultInfo info;
-    updated = cudaGraphExecUpdate(g.gexec, gr, &info) == cudaSuccess;
+    updated = g.cap_fns == g.gexec_fns && cudaGraphExecUpdate(g.gexec, gr, &info) == cudaSuccess;
     if (!updated) {
       cudaGetLastError();  // a structural mismatch is not an error: instantiate
       cudaGraphExecDestroy(g.gexec);
@@ -1212,6 +1221,7 @@ int launch_graph(cudaGraph_t gr, bc_batch_stats *st) {
   }
   cudaError_t e = updated ? cudaSuccess : cudaGraphInstantiate(&g.gexec, gr, 0);
   if (e != cudaSuccess) g.gexec = nullptr;
+  g.gexec_fns = g.cap_fns;
   cudaGraphDestroy(gr);
   CK(e);
   CK(cudaEventRecord(g.ev0, g.stream));
@@ -1497,6 +1507,8 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     if (!g.cap_stream) CK(cudaStreamCreateWithFlags(&g.cap_stream, cudaStreamNonBlocking));
     CK(cudaStreamBeginCapture(g.cap_stream, cudaStreamCaptureModeRelaxed));
     cap.s = lstream = g.cap_stream;
+    g.cap_fns.clear();
+    g.capturing = true;
   } else {
     CK(cudaEventRecord(g.ev0, g.stream));
   }
@@ -1551,6 +1563,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     p.carry_tiles = tiles;
     const ClassSlab &cs = slab[c.first];
     cudaStream_t cstream = nstreams ? g.class_stream[cls % nstreams] : lstream;
+    if (g.capturing) g.cap_fns.push_back(nullptr);
     if ((r = launch_class(s, sq, p, (long long)n, tiles, (double2 *)(base + cs.offA),
                           sq ? nullptr : (double2 *)(base + cs.offB), cstream, true, &st->launches,
                           b_late ? g.copy_ev[1] : nullptr, w16,
@@ -1566,6 +1579,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   if (graph) {
     cudaGraph_t gr = nullptr;
     cap.s = nullptr;
+    g.capturing = false;
     CK(cudaStreamEndCapture(g.cap_stream, &gr));
     if ((r = launch_graph(gr, st))) return r;
   }
