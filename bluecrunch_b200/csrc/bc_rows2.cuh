@@ -1,5 +1,5 @@
 // bc_rows2.cuh — the row pass for rows of P1 x P2 points (128, 192, 256, 320,
-// 384), each stage one transform in registers.
+// 384, 640, 768), each stage one transform in registers.
 //
 // Same arithmetic contract as k2_rows (bc_pipe.cuh): every row r of the class
 // gets A_r <- IDFT(DFT(A_r) . DFT(B_r)) (or the square), unscaled.  With
