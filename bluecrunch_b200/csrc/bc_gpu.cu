@@ -1232,6 +1232,20 @@ int launch_graph(cudaGraph_t gr, bc_batch_stats *st) {
   return BC_OK;
 }
 
+// An error between a batch's first launch and its outcomes: kernels already
+// launched end before the call returns, since they write their outcomes to
+// the pinned block that the next call uses.
+struct DrainGuard {
+  bool armed = true;
+  ~DrainGuard() {
+    if (!armed) return;
+    for (cudaStream_t s : g.class_stream)
+      if (s) cudaStreamSynchronize(s);
+    cudaStreamSynchronize(g.stream);
+    cudaGetLastError();
+  }
+};
+
 int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_stats *st, unsigned flags_in) {
   const bool all_host = flags_in & BC_BATCH_HOST_OPERANDS;
   const bool all_dev = flags_in & BC_BATCH_DEVICE_OPERANDS;
@@ -1498,6 +1512,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   // graph mode: every table exists before the capture (a new table's upload
   // synchronises the library stream), launches go to the capture stream
   cudaStream_t lstream = g.stream;
+  DrainGuard drain;  // declared before the capture's guard: that one ends first
   CaptureGuard cap;
   if (graph) {
     for (auto &c : classes) {
@@ -1597,6 +1612,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   // ---- outcomes, then outputs of the products that passed
   pt.next(&g_prof.wait);
   CK(cudaStreamSynchronize(g.stream));
+  drain.armed = false;
   std::vector<unsigned long long> errs(nw);
   std::vector<unsigned> flags(nw);
   for (size_t i = 0; i < nw; i++) {
