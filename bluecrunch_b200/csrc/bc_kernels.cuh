@@ -103,6 +103,11 @@ struct ClassParams {
   ItemDesc one;
 };
 
+// Limb words below digit n of an operand cut in digits of b bits, n a multiple
+// of 32.  Divided first: n b reaches 2^32 from transforms of 2^28 points on
+// (width 16), while n / 32 b stays below 2^30 for n up to 2^30 and b up to 24.
+__host__ __device__ __forceinline__ int words_below(int n, int b) { return n / 32 * b; }
+
 // What the outer forward pass reads of an item's operand, by value: from the
 // parameters' constant bank for a product alone in its call.
 struct FwdOperand {

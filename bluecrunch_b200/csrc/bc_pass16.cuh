@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(Fwd16<L, PARTS, TW>::NT, Fwd16<L, PARTS, TW>::
     const int XL = it.XL;
     const int b = it.b;
     const bool al16 = it.al16;
-    const int RW = (int)((unsigned)p.S1 * (unsigned)b / 32), PW = (int)((unsigned)p.M * (unsigned)b / 32);
+    const int RW = words_below(p.S1, b), PW = words_below(p.M, b);
     const int wbase = ((tl * W * b) >> 5) - 1 - seg_shift(tl, b, al16);
     const int parts = PARTS == 2 && it.nd > (unsigned)p.M ? 2 : 1;
     if (al16) {

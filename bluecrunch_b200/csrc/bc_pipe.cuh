@@ -557,11 +557,11 @@ __global__ void __launch_bounds__(PassTile<L>::NT, PassTile<L>::MINB) k2_outer_f
     const int tl = (int)f.rest;
     const FwdOperand it = fwd_operand(p, f.item, f.op);
     const uint32_t *X = it.X;
-    // word indices fit an int: operands and transforms stay below 2^29 words
+    // word indices fit an int: 2M digits of at most 24 bits are below 2^31 words
     const int XL = it.XL;
     const int b = it.b;
     const bool al16 = it.al16;
-    const int RW = (int)((unsigned)p.S1 * (unsigned)b / 32), PW = (int)((unsigned)p.M * (unsigned)b / 32);
+    const int RW = words_below(p.S1, b), PW = words_below(p.M, b);
     const int wbase = ((tl * W * b) >> 5) - 1 - seg_shift(tl, b, al16);
     uint32_t *dst = stg + st * K::STAGE_WORDS;
     // the imaginary parts hold digits M and up: none when nd <= M

@@ -1,0 +1,17 @@
+// Host-side check of the device index arithmetic (bc_kernels.cuh), compiled by
+// tests/test_index_logic.py with nvcc and run on the CPU.  Reads cases from
+// stdin and prints results for comparison with Python integers.
+#include <cstdio>
+#include "bc_kernels.cuh"
+using namespace bc;
+int main() {
+  char op[16];
+  while (scanf("%15s", op) == 1) {
+    if (op[0] == 'P') {  // P n b -> limb words below digit n
+      int n, b;
+      if (scanf("%d %d", &n, &b) != 2) return 1;
+      printf("%d\n", words_below(n, b));
+    }
+  }
+  return 0;
+}
