@@ -108,6 +108,10 @@ struct ClassParams {
 // (width 16), while n / 32 b stays below 2^30 for n up to 2^30 and b up to 24.
 __host__ __device__ __forceinline__ int words_below(int n, int b) { return n / 32 * b; }
 
+// Run records of a transform of M points: its 2M coefficients in runs of 8.
+// (2M itself does not fit an int at 2^30 points.)
+__host__ __device__ __forceinline__ unsigned long long run_records(int M) { return (unsigned long long)M / 4; }
+
 // What the outer forward pass reads of an item's operand, by value: from the
 // parameters' constant bank for a product alone in its call.
 struct FwdOperand {
@@ -462,7 +466,7 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
     const unsigned long long nruns = it.nruns, nwords = it.nwords;
     const int nr = (int)min((unsigned long long)CARRY_TILE_RUNS, nruns - rt);  // runs of this tile
     const int nbits = NB ? NB : 8 * it.b;
-    const unsigned long long nrec = (unsigned long long)(2 * p.M) / 8;
+    const unsigned long long nrec = run_records(p.M);
     const RunRec *const rec = it.rec + rt;
     // ---- records: run q*CARRY_NT + tid in slot q
     U192 h[CARRY_RPT];

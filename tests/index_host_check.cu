@@ -11,6 +11,10 @@ int main() {
       int n, b;
       if (scanf("%d %d", &n, &b) != 2) return 1;
       printf("%d\n", words_below(n, b));
+    } else if (op[0] == 'N') {  // N M -> run records of a transform
+      int M;
+      if (scanf("%d", &M) != 1) return 1;
+      printf("%llu\n", run_records(M));
     }
   }
   return 0;

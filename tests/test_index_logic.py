@@ -34,3 +34,10 @@ def test_words_below_the_imaginary_digits(checker):
     assert max(M for M, _ in cases) == 1 << 30
     for (M, b), line in zip(cases, run(checker, ["P %d %d" % c for c in cases])):
         assert int(line) == M * b // 32, (M, b)
+
+
+def test_run_records(checker):
+    # the carry pass looks for a carry out of the product at the last of them
+    cases = [M for M in bc.lengths() if M > 5120]
+    for M, line in zip(cases, run(checker, ["N %d" % M for M in cases])):
+        assert int(line) == 2 * M // 8, M
