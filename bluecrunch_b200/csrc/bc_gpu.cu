@@ -1232,13 +1232,16 @@ int launch_graph(cudaGraph_t gr, bc_batch_stats *st) {
   return BC_OK;
 }
 
-// An error between a batch's first launch and its outcomes: kernels already
-// launched end before the call returns, since they write their outcomes to
-// the pinned block that the next call uses.
+// An error between an attempt's first copy and its end: everything already
+// enqueued ends before the call returns.  Copies read and write the caller's
+// pinned arrays and the arena, and kernels write their outcomes to the pinned
+// block, all of which the next call uses.  copy_stream too: until the library
+// stream has waited for B's copy there, nothing else does.
 struct DrainGuard {
   bool armed = true;
   ~DrainGuard() {
     if (!armed) return;
+    if (g.copy_stream) cudaStreamSynchronize(g.copy_stream);
     for (cudaStream_t s : g.class_stream)
       if (s) cudaStreamSynchronize(s);
     cudaStreamSynchronize(g.stream);
@@ -1378,6 +1381,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
 
   // ---- inputs
   pt.next(&g_prof.copy_in);
+  DrainGuard drain;  // from the first copy on; declared before the capture's guard: that one ends first
   if (stage_in) {
     std::vector<SpanJob> jobs;  // in increasing span offset
     jobs.reserve(2 * nw);
@@ -1512,7 +1516,6 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   // graph mode: every table exists before the capture (a new table's upload
   // synchronises the library stream), launches go to the capture stream
   cudaStream_t lstream = g.stream;
-  DrainGuard drain;  // declared before the capture's guard: that one ends first
   CaptureGuard cap;
   if (graph) {
     for (auto &c : classes) {
@@ -1612,7 +1615,6 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
   // ---- outcomes, then outputs of the products that passed
   pt.next(&g_prof.wait);
   CK(cudaStreamSynchronize(g.stream));
-  drain.armed = false;
   std::vector<unsigned long long> errs(nw);
   std::vector<unsigned> flags(nw);
   for (size_t i = 0; i < nw; i++) {
@@ -1675,6 +1677,7 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
     g_prof.bytes_out += stage_out;
   }
   if (copies) CK(cudaStreamSynchronize(g.stream));
+  drain.armed = false;
   return BC_OK;
 }
 
