@@ -57,11 +57,12 @@ constexpr int kRowLens[] = {128, 192, 256, 320, 384, 512, 640, 768, 1024, 1280, 
 constexpr int kSmallLens[] = {256, 512, 768, 1024, 1280, 1536, 2048, 2560, 3072, 4096, 5120};
 constexpr int kOuterLens[] = {64, 128, 256, 512};
 constexpr size_t kMaxM = size_t(1) << 30;
-// Two levels up to this length, three above: two levels of 2^20 points and
-// more need rows of 2,560 to 4,096 points, which only the general row kernel
-// has.  Full-size products, two against three levels (ms): 2^19 0.067 / 0.076,
-// 3*2^18 0.089 / 0.085, 2^20 0.092 / 0.098, 5*2^18 0.129 / 0.113, 3*2^19
-// 0.149 / 0.121, 2^21 0.155 / 0.136.
+// Built-in number of levels: two up to this length, three above.  Rows of
+// 2,560 to 4,096 points, which only the general row kernel has, are what makes
+// two levels slow: full-size products, two against three levels (ms): 2^19
+// 0.067 / 0.076, 3*2^18 0.089 / 0.085, 2^20 0.092 / 0.098, 5*2^18 0.129 /
+// 0.113, 3*2^19 0.149 / 0.121, 2^21 0.155 / 0.136.  A line by length alone is a
+// compromise: three levels would win at 3*2^18 already (by 4 %).
 constexpr size_t kTwoLevelPoints = size_t(1) << 20;
 
 bool is_row_len(size_t L) {
@@ -71,7 +72,7 @@ bool is_row_len(size_t L) {
 size_t pow2part(size_t x) { return x & (~x + 1); }
 
 // The built-in decomposition of transform length M (shape_for below may
-// replace it by a tuned one with the same number of levels).
+// replace it by a tuned one).
 bool shape_default(size_t M, Shape &s) {
   if (M < 256 || M > kMaxM) return false;
   const size_t p2 = (M % 3 == 0) ? M / 3 : ((M % 5 == 0) ? M / 5 : M);
@@ -195,10 +196,11 @@ bool shape_for(size_t M, Shape &s) {
   return shape_default(M, s);
 }
 
-// Structural candidates for length M with as many levels as the built-in
-// shape: two levels L1 x Lr, three levels L1 x L2 x Lr, over the compiled
-// outer, middle and row lengths (launch consistency is checked separately,
-// shape_launch_ok).
+// Structural candidates for length M: the two-level splits L1 x Lr (above
+// kTwoLevelPoints they exist up to 2^21 points, behind the built-in three
+// levels), and where the built-in shape has three levels those L1 x L2 x Lr,
+// over the compiled outer, middle and row lengths (launch consistency is
+// checked separately, shape_launch_ok).
 std::vector<Shape> shape_candidates(size_t M) {
   std::vector<Shape> out;
   Shape d;
@@ -206,14 +208,12 @@ std::vector<Shape> shape_candidates(size_t M) {
   for (int L1 : kOuterLens) {
     if (M % L1) continue;
     const size_t R = M / L1;
-    if (d.levels == 2) {
-      if (is_row_len(R) && pow2part(R) >= (size_t)pass_tile_w(L1)) {
-        Shape s;
-        s.M = (int)M; s.L1 = L1; s.L2 = 1; s.Lr = (int)R; s.levels = 2;
-        out.push_back(s);
-      }
-      continue;
+    if (is_row_len(R) && pow2part(R) >= (size_t)pass_tile_w(L1)) {
+      Shape s;
+      s.M = (int)M; s.L1 = L1; s.L2 = 1; s.Lr = (int)R; s.levels = 2;
+      out.push_back(s);
     }
+    if (d.levels == 2) continue;
     for (int Lr : kRowLens) {
       if (R % Lr) continue;
       const size_t L2 = R / Lr;
