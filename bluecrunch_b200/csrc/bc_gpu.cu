@@ -1689,6 +1689,7 @@ int mul_batch_locked(const bc_mul_desc *items, size_t n, bc_batch_stats *st, Pla
   g_prof.calls++;
   std::vector<Work> works;
   works.reserve(n);
+  bool zeros_dev = false;
   PhaseTimer ppt(&g_prof.plan);
   for (size_t i = 0; i < n; i++) {
     const bc_mul_desc &d = items[i];
@@ -1697,9 +1698,12 @@ int mul_batch_locked(const bc_mul_desc *items, size_t n, bc_batch_stats *st, Pla
     if (d.CL == 0) continue;
     const bool zero = d.AL == 0 || d.BL == 0;
     if (zero) {
-      if ((flags & BC_BATCH_DEVICE_OPERANDS) || (!(flags & BC_BATCH_HOST_OPERANDS) && is_device_ptr(d.C)))
+      if ((flags & BC_BATCH_DEVICE_OPERANDS) || (!(flags & BC_BATCH_HOST_OPERANDS) && is_device_ptr(d.C))) {
         CK(cudaMemsetAsync(d.C, 0, d.CL * 4, g.stream));
-      else memset(d.C, 0, d.CL * 4);
+        zeros_dev = true;
+      } else {
+        memset(d.C, 0, d.CL * 4);
+      }
       continue;
     }
     Work w;
@@ -1710,6 +1714,7 @@ int mul_batch_locked(const bc_mul_desc *items, size_t n, bc_batch_stats *st, Pla
     works.push_back(w);
   }
   st->items = n;
+  if (zeros_dev && works.empty()) CK(cudaStreamSynchronize(g.stream));  // else the first attempt waits
   ppt.next(&g_prof_rest);  // the attempts are timed inside run_attempt
   if (g.time_kernels) g.ktimes.clear();
   // attempts: redo items whose rounding error reached the limit at a narrower width

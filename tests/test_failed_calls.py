@@ -83,3 +83,13 @@ for what in (COPY, LAUNCH):
         nth += 1
     assert fake.fake_pending() == 0 and fake.fake_calls(what) <= nth and (nth or what == COPY)
 """ % (kind, lens))
+
+
+def test_zeros_of_an_empty_operand_are_there_when_the_call_returns(fake):
+    _child(fake, """
+for other in ([], [(300, 200)]):
+    d = batch("device", [(0, 500)] + other)
+    fake.fake_fail(-1, 0)
+    assert lib.bc_gpu_mul_batch(d, len(d), None) == (-4 if other else 0)
+    assert fake.fake_pending() == 0, other
+""")
