@@ -1716,7 +1716,11 @@ int mul_batch_locked(const bc_mul_desc *items, size_t n, bc_batch_stats *st, Pla
   st->items = n;
   if (zeros_dev && works.empty()) CK(cudaStreamSynchronize(g.stream));  // else the first attempt waits
   ppt.next(&g_prof_rest);  // the attempts are timed inside run_attempt
-  if (g.time_kernels) g.ktimes.clear();
+  if (g.time_kernels) {
+    g.ktimes.clear();
+    for (auto e : g.kev) g.kev_pool.push_back(e);  // left by a call that failed
+    g.kev.clear();
+  }
   // attempts: redo items whose rounding error reached the limit at a narrower width
   for (int attempt = 0; attempt < 12; attempt++) {
     std::vector<Work *> todo;

@@ -93,3 +93,19 @@ for other in ([], [(300, 200)]):
     assert lib.bc_gpu_mul_batch(d, len(d), None) == (-4 if other else 0)
     assert fake.fake_pending() == 0, other
 """)
+
+
+def test_kernel_times_after_a_failed_call(fake):
+    # the failed call's events are not read with the next call's (there are
+    # no entries for them)
+    _child(fake, """
+d = batch("device", [(40000, 30000)])
+bc.time_kernels(True)
+assert call(d) == -4
+n = fake.fake_calls(LAUNCH)
+fake.fake_spans()
+assert call(d) == -4 and fake.fake_spans() == n + 1
+assert call(d, LAUNCH, n - 1) == -3 and fake.fake_spans() == 0
+assert call(d) == -4 and fake.fake_spans() == n + 1
+assert len(bc.kernel_times()) == n
+""")
