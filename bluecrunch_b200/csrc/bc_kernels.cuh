@@ -385,7 +385,7 @@ __device__ __forceinline__ U192 rec_h(const RunRec &r) { U192 h = {{r.h0, r.h1, 
 // for every word w that starts inside the run; a word that straddles into the
 // next run takes its high bits from `next`, that run's low 32 bits.
 template <class Put>
-__device__ __forceinline__ void run_words(unsigned long long bit0, int nbits, const U192 &h, uint32_t next,
+__host__ __device__ __forceinline__ void run_words(unsigned long long bit0, int nbits, const U192 &h, uint32_t next,
                                           const Put &put) {
   const unsigned long long w0 = (bit0 + 31) >> 5;
   const int o = (int)((w0 << 5) - bit0);  // bit of the run where word w0 starts, below 32

@@ -15,6 +15,14 @@ int main() {
       int M;
       if (scanf("%d", &M) != 1) return 1;
       printf("%llu\n", run_records(M));
+    } else if (op[0] == 'Q') {  // Q bit0 nbits h0 h1 h2 next -> "word value" of each word that starts in the run
+      unsigned long long bit0, h0, h1, h2;
+      int nbits;
+      unsigned next;
+      if (scanf("%llu %d %llx %llx %llx %x", &bit0, &nbits, &h0, &h1, &h2, &next) != 6) return 1;
+      const U192 h = {{h0, h1, h2}};
+      run_words(bit0, nbits, h, next, [](unsigned long long w, uint32_t x) { printf("%llu %x ", w, x); });
+      printf("\n");
     }
   }
   return 0;

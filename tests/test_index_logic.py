@@ -2,6 +2,7 @@
 headers and checked against Python integers for every transform length and
 digit width, the longest included."""
 import os
+import random
 import shutil
 import subprocess
 
@@ -41,3 +42,24 @@ def test_run_records(checker):
     cases = [M for M in bc.lengths() if M > 5120]
     for M, line in zip(cases, run(checker, ["N %d" % M for M in cases])):
         assert int(line) == 2 * M // 8, M
+
+
+def test_words_of_a_run(checker):
+    # every word that starts inside a run of 8 digits, the one that straddles
+    # into the next run with that run's low bits, at every digit width and at
+    # every place a run can have below a word boundary
+    rng = random.Random(11)
+    cases, want = [], []
+    for b in range(8, 25):
+        nbits = 8 * b
+        for r in list(range(40)) + [rng.randrange(1 << 28) for _ in range(40)]:
+            h = rng.choice([0, (1 << nbits) - 1, rng.randrange(1 << nbits)])
+            nxt = rng.choice([0, 0xFFFFFFFF, rng.randrange(1 << 32)])
+            bit0 = r * nbits
+            cases.append("Q %d %d %x %x %x %x" % (bit0, nbits, *((h >> s) & (2 ** 64 - 1) for s in (0, 64, 128)), nxt))
+            both = h | nxt << nbits
+            want.append([(w, both >> (32 * w - bit0) & 0xFFFFFFFF)
+                         for w in range((bit0 + 31) // 32, (bit0 + nbits + 31) // 32)])
+    for case, line, e in zip(cases, run(checker, cases), want):
+        f = line.split()
+        assert [(int(w), int(x, 16)) for w, x in zip(f[::2], f[1::2])] == e, case
