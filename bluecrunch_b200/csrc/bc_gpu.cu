@@ -643,7 +643,23 @@ int prepare(const KInfo &k, int *grid_cap) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.fn, k.threads, k.smem));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (n < 1) n = 1;
-    it = g_occ.emplace(std::make_pair(dev, k.fn), n * std::max(sms, 1)).first;
+    int ctas = n * std::max(sms, 1);
+    if (k.cluster > 1) {  // a cluster's CTAs share a GPC: fewer fit than CTAs alone
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = k.cluster;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(k.cluster);
+      cfg.blockDim = dim3(k.threads);
+      cfg.dynamicSmemBytes = k.smem;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      CK(cudaOccupancyMaxActiveClusters(&clusters, k.fn, &cfg));
+      ctas = std::max(1, clusters) * k.cluster;
+    }
+    it = g_occ.emplace(std::make_pair(dev, k.fn), ctas).first;
   }
   *grid_cap = it->second;
   return BC_OK;
@@ -794,12 +810,20 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
   bool pdl = false;
   if (!shape_launch_ok(s, sq)) return fail(BC_ERR_INVALID);
   if (s.levels == 1) {
-    // A cluster per product while the clusters are at most two waves of the
-    // SMs (one CTA per SM), one CTA per product above that: 32 products of
-    // 2,750 limbs (8 CTAs each) 47 against 58 us, 64 of them 70 against 57;
-    // 32 of 230 limbs 13 against 16 us, 64 of them 19 against 16.
+    // A cluster per product while the class is one round of the clusters that
+    // fit the GPU side by side (two rounds from 2,048 points on), else one CTA
+    // per product.  Kernel times in us, cluster / one CTA each, at the last
+    // count of a round and in the next one: 768 points 17.6 / 23.4 (30
+    // products), 25.3 / 23.5 (36); 1,024 points 16.6 / 19.9 (12), 22.4 / 21.7
+    // (24); 1,280 points 19.6 / 25.5 (30), 29.1 / 25.4 (36), 43.6 / 25.7 (72);
+    // two rounds (24) and three (36): 2,048 points 23.4 / 26.1, 35.8 / 27.1;
+    // 2,560 points 29.5 / 33.6, 48.3 / 33.6; 4,096 points 26.7 / 36.0, 41.9 /
+    // 35.9; 5,120 points 37.0 / 52.3, 62.7 / 52.3.
     const KInfo kc = get_cluster(s.M, sq);
-    return launch(n * kc.cluster <= 2 * g.sm_count ? kc : get_small(s.M, sq), n, params, nl, stream, timed);
+    int cap = 0;
+    if ((r = prepare(kc, &cap))) return r;
+    const long long round = std::max(1, cap / kc.cluster);
+    return launch(n <= round * (s.M >= 2048 ? 2 : 1) ? kc : get_small(s.M, sq), n, params, nl, stream, timed);
   }
   const cuuint64_t M16 = (cuuint64_t)s.M * 16, S1 = (cuuint64_t)params.S1, Lr = (cuuint64_t)params.Lr;
   const long long nfwd = n + (sq ? 0 : (long long)params.nb);  // forward operands

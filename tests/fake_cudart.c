@@ -85,7 +85,17 @@ cudaError_t cudaMemcpyAsync(void *d, const void *q, size_t n, enum cudaMemcpyKin
   return work(s, COPY);
 }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t s) { push(s, -1, 1); return cudaSuccess; }
-cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s) { return work(s, LAUNCH); }
+static int last_grid, clusters = 16;
+int fake_last_grid(void) { return last_grid; }
+void fake_clusters(int n) { clusters = n; }
+cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s) {
+  last_grid = g.x;
+  return work(s, LAUNCH);
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *f, const cudaLaunchConfig_t *c) {
+  *n = clusters;
+  return cudaSuccess;
+}
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **a) { return work(c->stream, LAUNCH); }
 cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s) {
   return work(s, LAUNCH);
