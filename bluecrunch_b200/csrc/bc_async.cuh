@@ -107,7 +107,13 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 // memory from read-only tables, then pdl_wait() blocks until the previous
 // grid has completed and its writes are visible (a no-op for a normal
 // launch).  Every global access to data another pass reads or writes comes
-// after it.  pdl_trigger() lets the next pass of the stream be launched.
+// after it, but for one: k_carry takes a tile from its counter before.
+// pdl_trigger() lets the next pass of the stream be launched.  A pass that is
+// not a class's first one waits before it triggers, always: then a pass that
+// runs knows all passes before the previous one complete, which k_carry's
+// counter (cleared by the first pass or before it) rests on.  A class has three
+// passes or more before the carry pass; the first, which triggers at once, is
+// launched normally.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <int N>

@@ -42,7 +42,11 @@ template <int M> struct ClusterShape {
   static constexpr int S = M / NC;           // row of one CTA
   static constexpr int P = S / NC;           // its share of the columns
   static constexpr int TC = S / PTS;         // threads of one row transform
-  static constexpr int NT = 2 * S < 512 ? 2 * S : 512;  // a point of A or B each, at most 128 registers
+  // a point of A or B each in the packing.  512 threads leave 128 registers,
+  // which the row transforms (NF threads) exceed where S is 3 or 5 times a
+  // power of two: 1,280, 1,536, 2,560, 3,072 and 5,120 points spill 160 to 350
+  // bytes a thread, 768 points (384 threads) 88.
+  static constexpr int NT = 2 * S < 512 ? 2 * S : 512;
   static constexpr int NF = (2 * TC + 31) / 32 * 32;    // threads that run the row transforms
   static constexpr int NG = (NF + TC - 1) / TC;  // their groups (two in use, the rest idle along)
   static constexpr int SEG = 2 * NC;         // segments of the product per CTA

@@ -525,7 +525,8 @@ __host__ __device__ __forceinline__ bool u192_is_ones(const U192 &h, int nbits) 
   return h.w[0] == ~0ull && h.w[1] == m1 && h.w[2] == m2;
 }
 
-// Bits [off, off+32) of a 192-bit value (off may exceed 192 -> 0).
+// Bits [off, off+32) of a 192-bit value (off may exceed 192 -> 0).  No kernel
+// needs it (run_words); the host-side check of the tests does.
 __host__ __device__ __forceinline__ uint32_t u192_bits32(const U192 &h, int off) {
   if (off >= 192) return 0;
   const int wi = off >> 6, bi = off & 63;

@@ -1375,7 +1375,8 @@ int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_s
       status_words += pl.ntiles;
     }
   }
-  // err, flags, counters and status words: one region, cleared by one memset
+  // err, flags, counters and status words: one region, cleared by the first
+  // kernel of a lone product, else by the copy of the descriptors or a memset
   const size_t off_err = off; off += align256(nw * 8);
   const size_t off_flags = off; off += align256(nw * 4);
   const size_t off_ctr = off; off += 256 * (classes.size() + 1);
@@ -1797,7 +1798,7 @@ int mul_batch_locked(const bc_mul_desc *items, size_t n, bc_batch_stats *st, Pla
 // Binary splitting of sum 1/k! with every value kept in device memory: the
 // leaves (LEAF_TERMS terms each) by k_bsr_leaves, then one level at a time
 // the products P_l*Q_r and Q_l*Q_r of neighbouring nodes in one batch
-// (device operands), their lengths by k_trim and P = P_l*Q_r + P_r by k_add.
+// (device operands), then P = P_l*Q_r + P_r and the products' lengths by k_add.
 // Only the lengths cross to the host between steps; P and Q of the root at
 // the end.
 struct DevNum {

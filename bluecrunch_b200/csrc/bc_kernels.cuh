@@ -201,13 +201,6 @@ __device__ __forceinline__ unsigned fwd_units_b(const ClassParams &p, unsigned p
   return (!p.sq && p.fwd_ops != 1) ? (unsigned)p.nb * per_op : 0u;
 }
 
-// e^{-2 pi i m/(4M)} for m = s*(4k-1) with s < S, k < 4M/(4S): m < 4M when
-// k >= 1; for k = 0 it is the conjugate of m = s.
-__device__ __forceinline__ double2 outer_tw(const Tw2 &T, int s, int k) {
-  if (k == 0) { double2 w = tw2_get(T, (uint64_t)s); return make_double2(w.x, -w.y); }
-  return tw2_get(T, (uint64_t)s * (uint64_t)(4 * k - 1));
-}
-
 // Nearest integer of |z| < 2^51 (ties to even, as rint): added to 1.5 2^52 the
 // fraction is rounded off.  Above that the result stays near z, so the check
 // below still sees a value too large.
@@ -371,8 +364,8 @@ __device__ __forceinline__ uint32_t block_scan_fn(uint32_t f, uint32_t *sw, uint
 // without ordering other memory.
 // What bounds it: HBM, 32 bytes read and b bytes written per run.  Staging
 // each tile in shared memory, scanning every tile and looking back for every
-// one (7 to 11 barrier stalls an issue) took 0.138 ms for the 2^24-limb
-// product's 2^26 coefficients (2.9 TB/s); this form takes 0.070 ms (5.8 TB/s).
+// one took 0.138 ms for the 2^24-limb product's 2^26 coefficients (2.9 TB/s);
+// this form takes 0.070 ms (5.8 TB/s).
 constexpr int CARRY_NT = 256;
 constexpr int CARRY_RPT = 4;                            // runs per thread, CARRY_NT apart
 constexpr int CARRY_TILE_RUNS = CARRY_NT * CARRY_RPT;   // runs per tile
@@ -446,6 +439,9 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
   __shared__ uint32_t sw[65];
   __shared__ unsigned s_unit[2];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  // Before the wait: the counter was cleared two or more launches ago (by the
+  // class's first kernel or a copy before it), and every pass between waits
+  // before it triggers, so what came before the previous pass is complete here.
   if (tid == 0) s_unit[0] = atomicAdd(p.counter, 1u);
   pdl_wait();
   pdl_trigger();
@@ -624,7 +620,7 @@ __global__ void __launch_bounds__(CARRY_NT, 4) k_carry(ClassParams p) {
 }
 
 // ------------------------------------------------------------------ small
-// Whole product in one CTA of M/8 threads (M <= 4096): pack, FFT, product,
+// Whole product in one CTA of M/8 threads (M <= 5120): pack, FFT, product,
 // inverse, round, runs, in-CTA carry scan, words.
 template <int M, bool SQ>
 __global__ void __launch_bounds__(M / PTS, 1) k_small(ClassParams p) {

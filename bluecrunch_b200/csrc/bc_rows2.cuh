@@ -9,9 +9,10 @@
 //            thread k1 (< P1): DFT-P2 over j: X[k1 + P1 k2] in w[k2].
 //   inverse  the same steps backwards: thread k1 inverse DFT-P2, exchange,
 //            thread j conjugate twiddle, inverse DFT-P1, points j + P2 i.
-// A and B meet in registers, B's spectrum stays there while A is transformed.
-// A row is held by max(P1, P2) threads; rows of 16 threads are private to a
-// warp (two of them), others synchronise over the CTA.
+// A and B meet in registers.  Up to 256 points B's spectrum stays there while A
+// is transformed, from 320 on it waits in B's buffer.  A row is held by
+// max(P1, P2) threads; rows whose threads divide a warp (16 of them up to 256
+// points, 32 at 640 and 768) are private to it, others synchronise over the CTA.
 //
 // What bounds it: shared memory and FP64 about alike.  k2_rows exchanges two
 // or three times per transform (and stores the odd radix's points back
@@ -81,7 +82,8 @@ template <int L> struct Rows2 {
   static constexpr int ROW = (P1 * PITCH > L ? P1 * PITCH : L);  // entries of a row's buffer
   // ten or twelve warps per SM, at most 168 registers (640 and 768 points:
   // eight, 255); B's spectrum stays in registers where that leaves room, else
-  // in B's buffer
+  // in B's buffer.  168 are too few for 384 points, which spill 228 bytes a
+  // thread (squares 116); 192 points spill 32, the others nothing.
   static constexpr int MINB = L == 768 ? 1 : (L == 640 || NT != 128 ? 2 : 3);
   static constexpr bool PARK = L >= 320;
   static constexpr size_t SMEM = (size_t)(2 * NR * ROW + L) * 16;

@@ -61,11 +61,11 @@ __device__ __forceinline__ void row_dft512(double2 (&v)[R5_P], int lane, double2
   dft16<INV>(v);  // over l1: v[k2'] = X[lane + 32 k2']
 }
 
-// What bounds it: shared memory (0.75 of the LSU data path's rate: per row and
-// transform one read of the row, the twiddles, the transpose's write and twice
-// its read).  So B's spectrum stays in registers while A is transformed (255
-// of them, no spills; parked in shared memory it cost 128 of 1,166 passes per
-// row: 0.343 -> 0.334 ms at 2^25 points).  Two CTAs of four warps share an SM;
+// What bounds it: shared memory (943 passes over its data path per row, 0.72 of
+// that unit's rate: per row and transform one read of the row, the twiddles,
+// the transpose's write and twice its read).  So B's spectrum stays in
+// registers while A is transformed (255 of them, 12 bytes spilled; parked in
+// shared memory it took 0.343 ms at 2^25 points instead of 0.334).  Two CTAs of four warps share an SM;
 // three (168 registers) or two of five measured the same or slower.  Loading 6
 // of the 15 twiddles and multiplying the others took 0.331 ms, but raised the
 // rounding error of 2^18-point products by a tenth.

@@ -83,7 +83,7 @@ typedef struct {
 typedef struct {
   size_t fft_points;      /* M */
   int width;              /* b */
-  int levels;             /* 1 = single-CTA kernel, 2 or 3 = passes over HBM */
+  int levels;             /* 1 = one kernel (a CTA or a cluster), 2 or 3 = passes over HBM */
   int L1, L2, Lr;         /* decomposition M = L1 * L2 * Lr (L2 = 1 for two levels) */
   size_t digits_a, digits_b;
   size_t out_words;       /* words produced by the transform (the rest are 0) */
