@@ -1273,6 +1273,13 @@ struct DrainGuard {
   }
 };
 
+// The same for calls of several steps: their copies use the pinned ring, the
+// caller's arrays and scratch that the next call takes.
+int settle(int r) {
+  if (r != BC_OK && g.init) DrainGuard();
+  return r;
+}
+
 int run_attempt(const bc_mul_desc *items, std::vector<Work *> &works, bc_batch_stats *st, unsigned flags_in) {
   const bool all_host = flags_in & BC_BATCH_HOST_OPERANDS;
   const bool all_dev = flags_in & BC_BATCH_DEVICE_OPERANDS;
@@ -2923,31 +2930,31 @@ int bc_gpu_e_series(uint32_t a, uint32_t b, uint32_t **P, size_t *PL, uint32_t *
   std::lock_guard<std::recursive_mutex> lk(g_mu);
   bc_batch_stats st{};
   *P = *Q = nullptr;
-  return e_series_locked(a, b, P, PL, Q, QL, &st);
+  return settle(e_series_locked(a, b, P, PL, Q, QL, &st));
 }
 
 int bc_gpu_radix_tree(const uint32_t *y, size_t ylen, const bc_radix_node *nodes, size_t nnodes,
                       const uint32_t *const *table, const size_t *table_len, int ntable, double alpha,
                       uint32_t *out) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
-  return radix_tree_locked(y, ylen, nodes, nnodes, table, table_len, ntable, alpha, out);
+  return settle(radix_tree_locked(y, ylen, nodes, nnodes, table, table_len, ntable, alpha, out));
 }
 
 int bc_gpu_radix_tree_pow(const uint32_t *y, size_t ylen, const bc_radix_node *nodes, size_t nnodes,
                           const uint32_t *t0, size_t t0len, const bc_radix_pow_step *steps, int ntable, double alpha,
                           uint32_t *out) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
-  return radix_tree_pow_locked(y, ylen, nodes, nnodes, t0, t0len, steps, ntable, alpha, out);
+  return settle(radix_tree_pow_locked(y, ylen, nodes, nnodes, t0, t0len, steps, ntable, alpha, out));
 }
 
 int bc_gpu_mul_small_batch(const bc_mul_desc *items, size_t n) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
-  return mul_small_locked(items, n);
+  return settle(mul_small_locked(items, n));
 }
 
 int bc_gpu_decimal_write(const uint32_t *limbs, size_t top, size_t n, size_t maxbytes, int fd, long long offset) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
-  return decimal_write_locked(limbs, top, n, maxbytes, fd, offset);
+  return settle(decimal_write_locked(limbs, top, n, maxbytes, fd, offset));
 }
 
 int bc_gpu_device_alloc(size_t bytes, void **p) {
@@ -2990,12 +2997,12 @@ int bc_gpu_selftest_wait(double *seconds) {
 int bc_gpu_newton(const bc_bignum *den, const bc_bignum *r0, const size_t *levels, int nlevels, const bc_bignum *num,
                   size_t pdiv, bc_bignum_out *out) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
-  return newton_locked(den, r0, levels, nlevels, num, pdiv, out);
+  return settle(newton_locked(den, r0, levels, nlevels, num, pdiv, out));
 }
 
 int bc_gpu_radix_leaves(const bc_radix_leaf *leaves, size_t count, double alpha) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
-  return radix_leaves_locked(leaves, count, alpha);
+  return settle(radix_leaves_locked(leaves, count, alpha));
 }
 
 int bc_gpu_set_stream(void *stream) {
@@ -3240,6 +3247,11 @@ extern "C" int bc_gpu_mul_noalloc(uint32_t *C, size_t CL, const uint32_t *A, siz
   if (std::min(AL, CL) + std::min(BL, CL) > kNoAllocMaxLimbs) return fail(BC_ERR_TOO_LARGE);
   const bool square = A == B && AL == BL;
   int bcap = 24;
+  struct Drain {  // an error between the steps: what is enqueued ends first (the next call may come on another stream)
+    cudaStream_t s;
+    bool armed = true;
+    ~Drain() { if (armed) cudaStreamSynchronize(s); }
+  } drain{stream};
   for (int attempt = 0; attempt < 12; attempt++) {
     Plan pl;
     if (!make_plan(AL, BL, CL, square, bcap, pl, kNoAllocMaxPoints))
@@ -3299,11 +3311,13 @@ extern "C" int bc_gpu_mul_noalloc(uint32_t *C, size_t CL, const uint32_t *A, siz
     CK(cudaMemcpyAsync(&errbits, it.err, 8, cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync(&flags, it.flags, 4, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
+    drain.armed = false;
     if (flags & FLAG_TIMEOUT) return fail(BC_ERR_TIMEOUT);
     double e;
     memcpy(&e, &errbits, 8);
     if (e < g.max_err && !(flags & FLAG_TOPCARRY)) return BC_OK;
     bcap = pl.b - 1;  // narrower digits, as bc_gpu_mul retries
+    drain.armed = true;
   }
   return fail(BC_ERR_PRECISION);
 }

@@ -14,7 +14,17 @@ void fake_fail(int kind, int nth) {
   if (kind >= 0) fail_at[kind] = nth;
 }
 int fake_calls(int kind) { return calls[kind]; }
-static int fails(int kind) { return calls[kind]++ == fail_at[kind]; }
+static cudaError_t last_error;
+static int fails(int kind) {
+  if (calls[kind]++ != fail_at[kind]) return 0;
+  last_error = cudaErrorUnknown;
+  return 1;
+}
+cudaError_t cudaGetLastError(void) {
+  cudaError_t e = last_error;
+  last_error = cudaSuccess;
+  return e;
+}
 
 /* ---- operations in flight */
 typedef struct { int prev, dep, done, work; } Op;
@@ -106,6 +116,17 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *f,
   return cudaSuccess;
 }
 
+/* a <<<>>> launch: its shape, then cudaLaunchKernel */
+static struct { dim3 g, b; size_t m; cudaStream_t s; } cfg;
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t m, struct CUstream_st *s) {
+  cfg.g = g; cfg.b = b; cfg.m = m; cfg.s = s;
+  return 0;
+}
+cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *m, void *s) {
+  *g = cfg.g; *b = cfg.b; *m = cfg.m; *(cudaStream_t *)s = cfg.s;
+  return cudaSuccess;
+}
+
 /* ---- streams and events */
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) {
   *s = malloc(sizeof **s);
@@ -139,7 +160,7 @@ cudaError_t cudaGetDeviceProperties(struct cudaDeviceProp *p, int d) {
   return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d) { *v = 148; return cudaSuccess; }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetSymbolAddress(void **p, const void *v) { return take(p, 16 << 20, cudaMemoryTypeDevice); }
 const char *cudaGetErrorString(cudaError_t e) { return "made by the test"; }
 static int encode_tensor_map() { return 0; }
 cudaError_t cudaGetDriverEntryPointByVersion(const char *n, void **f, unsigned v, unsigned long long fl,

@@ -109,3 +109,48 @@ assert call(d, LAUNCH, n - 1) == -3 and fake.fake_spans() == 0
 assert call(d) == -4 and fake.fake_spans() == n + 1
 assert len(bc.kernel_times()) == n
 """)
+
+
+@pytest.mark.parametrize("what", ["small", "leaves", "series", "text", "noalloc"])
+def test_nothing_in_flight_after_other_failing_calls(fake, what):
+    # every copy and launch of these calls fails in turn; without kernels their
+    # results mean nothing, so any end that is not a CUDA error will do
+    _child(fake, """
+what = %r
+lib.bc_gpu_mul_noalloc.argtypes = None
+if what == "small":
+    d = batch("pageable", [(100, 90)] * 40)
+    f = lambda: lib.bc_gpu_mul_small_batch(d, len(d))
+elif what == "leaves":
+    import numpy as np
+    class Leaf(ctypes.Structure):
+        _fields_ = [("y", ctypes.c_void_p), ("len", ctypes.c_size_t), ("n", ctypes.c_size_t), ("k", ctypes.c_size_t),
+                    ("s", ctypes.c_void_p)]
+    l = (Leaf * 3)(*[Leaf(memory("pageable", 50), 50, 50, 40, memory("pageable", 40)) for _ in range(3)])
+    f = lambda: lib.bc_gpu_radix_leaves(ctypes.cast(l, ctypes.c_void_p), 3, ctypes.c_double(0.93))
+elif what == "series":
+    p, q = ctypes.POINTER(ctypes.c_uint32)(), ctypes.POINTER(ctypes.c_uint32)()
+    pl, ql = ctypes.c_size_t(), ctypes.c_size_t()
+    f = lambda: lib.bc_gpu_e_series(0, 5000, ctypes.byref(p), ctypes.byref(pl), ctypes.byref(q), ctypes.byref(ql))
+elif what == "text":
+    import os
+    fd = os.open("/dev/null", os.O_WRONLY)
+    x = memory("pageable", 5000)
+    f = lambda: lib.bc_gpu_decimal_write(ctypes.c_void_p(x), ctypes.c_size_t(4999), ctypes.c_size_t(5000),
+                                         ctypes.c_size_t(45000), fd, ctypes.c_longlong(0))
+else:
+    c, a, b = memory("device", 9000), memory("device", 5000), memory("device", 4000)
+    S = ctypes.c_size_t
+    f = lambda: lib.bc_gpu_mul_noalloc(ctypes.c_void_p(c), S(9000), ctypes.c_void_p(a), S(5000), ctypes.c_void_p(b),
+                                       S(4000), None)
+failed = 0
+for kind in (COPY, LAUNCH):
+    for nth in range(40):
+        fake.fake_fail(kind, nth)
+        r = f()
+        failed += r == -3
+        assert r == -3 or fake.fake_calls(kind) <= nth, (kind, nth, r)
+        if r == -3:
+            assert fake.fake_pending() == 0, (kind, nth, fake.fake_pending())
+assert failed >= 2, failed
+""" % what)
