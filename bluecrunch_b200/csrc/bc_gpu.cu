@@ -820,10 +820,13 @@ int launch_class(const Shape &s, bool sq, const ClassParams &params, long long n
     // 2,560 points 29.5 / 33.6, 48.3 / 33.6; 4,096 points 26.7 / 36.0, 41.9 /
     // 35.9; 5,120 points 37.0 / 52.3, 62.7 / 52.3.
     const KInfo kc = get_cluster(s.M, sq);
-    int cap = 0;
-    if ((r = prepare(kc, &cap))) return r;
-    const long long round = std::max(1, cap / kc.cluster);
-    return launch(n <= round * (s.M >= 2048 ? 2 : 1) ? kc : get_small(s.M, sq), n, params, nl, stream, timed);
+    bool fits = n == 1;  // without a look-up: it is the shortest calls' path
+    if (!fits) {
+      int cap = 0;
+      if ((r = prepare(kc, &cap))) return r;
+      fits = n <= std::max(1, cap / kc.cluster) * (s.M >= 2048 ? 2 : 1);
+    }
+    return launch(fits ? kc : get_small(s.M, sq), n, params, nl, stream, timed);
   }
   const cuuint64_t M16 = (cuuint64_t)s.M * 16, S1 = (cuuint64_t)params.S1, Lr = (cuuint64_t)params.Lr;
   const long long nfwd = n + (sq ? 0 : (long long)params.nb);  // forward operands
